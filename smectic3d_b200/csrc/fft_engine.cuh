@@ -263,11 +263,25 @@ __device__ constexpr double kSin16[8] = {0.0, 0.38268343236508977173, 0.70710678
                                           0.92387953251128675613, 1.0, 0.92387953251128675613,
                                           0.70710678118654752440, 0.38268343236508977173};
 
+// cos / sin of 2 pi a / 32, odd a
+__device__ constexpr double kCos32[16] = {0, 0.98078528040323044913, 0, 0.83146961230254523708,
+                                           0, 0.55557023301960222474, 0, 0.19509032201612826785,
+                                           0, -0.19509032201612826785, 0, -0.55557023301960222474,
+                                           0, -0.83146961230254523708, 0, -0.98078528040323044913};
+__device__ constexpr double kSin32[16] = {0, 0.19509032201612826785, 0, 0.55557023301960222474,
+                                           0, 0.83146961230254523708, 0, 0.98078528040323044913,
+                                           0, 0.98078528040323044913, 0, 0.83146961230254523708,
+                                           0, 0.55557023301960222474, 0, 0.19509032201612826785};
+
 // multiply by w_R^k = exp(DIR * 2 pi i k / R), 0 <= k < R/2
 template <typename T, int R, int K, int DIR>
 __device__ __forceinline__ cplx<T> twc(cplx<T> v) {
-  constexpr int A = K * (16 / R);  // angle in units of 2 pi / 16, < 8
-  if constexpr (A == 0) {
+  constexpr int A = R == 32 ? K / 2 : K * (16 / R);  // angle in units of 2 pi / 16, < 8
+  if constexpr (R == 32 && K % 2 == 1) {
+    const T c = T(kCos32[K]);
+    const T s = DIR < 0 ? T(-kSin32[K]) : T(kSin32[K]);
+    return mk<T>(fma(v.x, c, -v.y * s), fma(v.x, s, v.y * c));
+  } else if constexpr (A == 0) {
     return v;
   } else if constexpr (A == 4) {
     // w = DIR * i

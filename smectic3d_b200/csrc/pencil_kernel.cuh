@@ -1,31 +1,26 @@
 // Pencil pass: the x transform, fused with the spectral time update.
 //
 // A CTA owns TK consecutive in-plane positions f (128 bytes of every x-plane
-// row, so each x step is one coalesced segment) and all N values of x.  The
-// forward x transform completes the 3-D spectrum of the nonlinear term; the
-// CNAB2 update runs in registers; the inverse x transform of the new psi
-// spectrum starts from the same registers (the inverse radix plan is the
-// forward plan reversed).
+// row) and all N values of x.  Lanes run along f, so every global access of a
+// warp is whole 128-byte row segments straight between HBM and registers: no
+// staging of the tile in shared memory, which only carries the one exchange
+// between the two register passes of each transform (line_fft.cuh).  A thread
+// holds wavenumbers k and N - k together, so the cosine transforms pair them in
+// registers.  The forward x transform completes the 3-D spectrum of the
+// nonlinear term; the CNAB2 update runs in registers; the inverse x transform
+// of the new psi spectrum starts from the same registers.
 //
-// The spectral state is W^n = C1 psihat^n - dt/2 Nhat^{n-1}, stored
-// pencil-major ([f][kx], kx contiguous) so that each thread's register slots
-// map to coalesced addresses.  The reference update
+// The spectral state is W^n = C1 psihat^n - dt/2 Nhat^{n-1}, stored like the
+// partials, [kx][f].  The reference update
 //   psihat^{n+1} = (C1 psihat^n + dt/2 (3 Nhat^n - Nhat^{n-1})) / C2
 // (periodicFFT/pf3d.cpp:476-478, cosFFT/mesabi/cosNoAdvMorph.cpp:524-525)
 // becomes psihat^{n+1} = (W^n + 3 dt/2 Nhat^n) / C2 and
-// W^{n+1} = C1 psihat^{n+1} - dt/2 Nhat^n: one state read and one write.
+// W^{n+1} = C1 psihat^{n+1} - dt/2 Nhat^n: one state read and one state write.
 #pragma once
+#include "line_fft.cuh"
 #include "sh_common.cuh"
 
 namespace shb {
-
-// warps per SM the FP32 step kernels are register-budgeted for
-#ifndef SHB_STEP_WARPS
-#define SHB_STEP_WARPS 24
-#endif
-#ifndef SHB_STEP_WARPS_F64
-#define SHB_STEP_WARPS_F64 16
-#endif
 
 enum PencilMode : int {
   kPencilStep = 0,
@@ -36,11 +31,13 @@ enum PencilMode : int {
   kPencilInitAdv = 4,
   kPencilStokes = 5,   // Stokes velocity from the stress (periodicFFT/pf3d.cpp:433-447)
   kPencilXMul = 6,     // partial P -> partial of its spectrum times an x-line multiplier (XMul)
-  kPencilSpec = 7,     // partial P -> psihat, pencil-major
+  kPencilSpec = 7,     // partial P -> psihat
   kPencilAdjInit = 8,  // adjoint: partial of lambda^T -> lambdahat^T, mu partial
   kPencilAdj = 9,      // adjoint step: lambdahat^n = A lambdahat^{n+1} + ghat^n, mu partial, parameter gradients
   kPencilAdjOut = 10,  // adjoint: lambdahat -> its x-inverse partial (for lambda^0 in real space)
   kPencilStepU64 = 11, // the step of FP32 fields with the CNAB2 multipliers and update in FP64
+  kPencilStepGen = 12, // the step with what kPencilStep leaves out: IMEX Euler, the energy, psihat out
+  kPencilStepU64Gen = 13,  // the same for kPencilStepU64
 };
 // multiplier of kPencilXMul
 enum XMulKind : int {
@@ -50,25 +47,26 @@ enum XMulKind : int {
   kXSinDx = 3,   // Neumann: x derivative of the cosine series, as the reversed coefficients
                  // -q_{N-k} X[N-k] (0 at k = 0) whose REDFT01 is (-1)^x psi_x
 };
-// line sets of shared memory a pencil mode uses (FFT scratch, stash, Stokes components)
+// tiles of shared memory a pencil mode uses (the exchange, a spectrum kept
+// aside, Stokes components)
 __host__ __device__ constexpr int pencil_sets(int mode) {
-  return mode == kPencilStokes ? 3 : ((mode == kPencilStepAdv || mode == kPencilInitAdv) ? 2 : 1);
+  return mode == kPencilStokes ? 3 : ((mode == kPencilStepAdv || mode == kPencilInitAdv || mode == kPencilInit) ? 2 : 1);
 }
 
 // TKV: lines per CTA (the tile), 0 = the default of 16 (FP32) or 8 (FP64)
 template <typename T, int N, bool DCT, int TKV = 0>
 struct PencilCfg {
-  static constexpr int E = Plan<N>::E;
-  static constexpr int G = N / E;
-  static constexpr int TK = TKV > 0 ? TKV : (sizeof(T) == 4 ? 16 : 8);
+  using I = LineIdx<N>;
+  static constexpr int E = I::E;
+  static constexpr int G = I::G;
+  // 128-byte row segments; at least one warp per CTA
+  static constexpr int TK_DEF = sizeof(T) == 4 || N < 32 ? 16 : 8;
+  static constexpr int TK = TKV > 0 ? TKV : TK_DEF;
   static constexpr int THREADS = TK * G;
-  static constexpr int LS = line_stride(N);
   static constexpr int FP = DCT ? N * (N / 2) : N * (N / 2 + 1);
   static constexpr int TILES = FP / TK;
-  static constexpr int RL = radix_of<N, -1, Plan<N>::P - 1>();
-  static constexpr size_t SET_BYTES = size_t(TK) * LS * sizeof(cplx<T>);
-  static constexpr size_t tw_off(int mode) { return SET_BYTES * pencil_sets(mode); }
-  static constexpr size_t red_off(int mode) { return tw_off(mode) + size_t(tw_staged<N>(DCT)) * sizeof(cplx<T>); }
+  static constexpr size_t SET_BYTES = size_t(TK) * N * sizeof(cplx<T>);
+  static constexpr size_t red_off(int mode) { return SET_BYTES * pencil_sets(mode); }
   // |k| shells of the spectral-power histogram (shell = rint |index vector|):
   // at most sqrt(3) N / 2 + 1 periodic, sqrt(3) (N - 1) + 1 Neumann
   static constexpr int NSHELL = DCT ? 2 * N : N;
@@ -76,20 +74,24 @@ struct PencilCfg {
   static constexpr size_t smem(int mode) {
     return shell_off(mode) + (mode == kPencilEnergy ? size_t(NSHELL) * sizeof(double) : 0);
   }
-  // per-CTA shared memory limit of sm_100 (the Stokes mode's three line sets
-  // do not fit at 512^3 in FP64)
+  // per-CTA shared memory limit of sm_100
   static constexpr bool fits(int mode) { return smem(mode) <= size_t(227) * 1024; }
-  // The step asks ptxas for a register budget that keeps SHB_STEP_WARPS warps
-  // per SM resident in FP32 (three 256-thread CTAs at 256^3, twelve 64-thread
-  // CTAs at 64^3) and SHB_STEP_WARPS_F64 in FP64 at N <= 128; every other
-  // launch leaves the register budget to ptxas (0).
-  // FP64 holds twice the registers per value: only its small CTAs (N <= 128) get a budget
-  static constexpr int step_warps() { return sizeof(T) == 4 ? SHB_STEP_WARPS : (THREADS <= 64 ? SHB_STEP_WARPS_F64 : 0); }
-  static constexpr int min_blocks(int mode) {
-    return ((mode == kPencilStep || mode == kPencilStepU64) && THREADS <= 256 && step_warps() * 32 / THREADS >= 2)
-               ? step_warps() * 32 / THREADS
-                                                                                      : 0;
+  // Threads per SM that the register budget aims at: the E values of a thread, the
+  // values read ahead and the temporaries of a radix-16 butterfly, without spills.
+  // FP32 at 256^3: 384 threads (168 registers, three CTAs) and 512 (128 registers,
+  // 8 bytes of spills) measure the same, 63.4 and 64.3 us.  FP32, E = 16: 768
+  // threads periodic (64 x 64^3: 52.8 us, with 512 55.5), 512 Neumann, whose pairing
+  // spills at 80 registers (57.0 us, with 768 60.6).
+  static constexpr int step_threads() {
+    return sizeof(T) == 4 ? (E == 32 ? 384 : (DCT ? 512 : 768)) : (E == 32 ? 256 : 512);
   }
+  static constexpr int min_blocks(int mode) {
+    return mode != kPencilInit && mode != kPencilInitAdv && mode != kPencilEnergy && step_threads() >= THREADS
+               ? step_threads() / THREADS
+               : 0;
+  }
+  // values of W (or of the adjoint's fields) a thread reads ahead of the update
+  static constexpr int WB = E < 16 ? E : (sizeof(T) == 4 && (E == 32 || DCT) ? 16 : 8);
   static_assert(FP % TK == 0, "tile must divide the plane");
   static_assert(THREADS % 32 == 0, "pencil CTA must be whole warps");
 };
@@ -98,13 +100,13 @@ template <typename T>
 struct PencilArgs {
   const cplx<T>* src;   // step: partial of N ; init: partial of psi   [rep][x][FP]
   const cplx<T>* src2;  // init: partial of N(psi)
-  cplx<T>* w;           // state W [rep][FP][N]
+  cplx<T>* w;           // state W [rep][kx][FP] (adjoint: lambdahat)
   cplx<T>* dst;         // partial of scale * psihat^{n+1}, x-inverse applied [rep][x][FP]
   cplx<T>* dst_x;       // advection: partial of scale * i q_x psihat^{n+1}
   cplx<T>* dst_sh;      // advection: partial of scale * opSH psihat^{n+1}
-  cplx<T>* spec_out;     // kFlSpecOut / kPencilSpec: psihat, pencil-major
-  const cplx<T>* spec_a; // adjoint: psihat^n, pencil-major
-  const cplx<T>* spec_b; // adjoint: psihat^{n+1}, pencil-major
+  cplx<T>* spec_out;     // kFlSpecOut / kPencilSpec: psihat [rep][kx][FP]
+  const cplx<T>* spec_a; // adjoint: psihat^n [rep][kx][FP]
+  const cplx<T>* spec_b; // adjoint: psihat^{n+1} [rep][kx][FP]
   const cplx<T>* s3[3]; // Stokes: partial stress components (forward y,z applied)
   cplx<T>* u3[3];       // Stokes: partial velocity components (may alias s3)
   double* red;          // per-CTA spectral energy partial [rep][grid.x]
@@ -114,7 +116,9 @@ struct PencilArgs {
   int xmul;             // kPencilXMul: XMulKind
   const T* q;           // wavenumber table (N entries)
   const double* qd;     // the same wavenumbers in FP64
-  const cplx<T>* tw;    // twiddle table [forward | inverse | quarter-wave]
+  const T* qs;          // q of every B-side slot [t][E] (canonical order for the cosine transforms)
+  const double* qds;    // qd of every B-side slot [t][E]
+  const cplx<T>* lt;    // line tables (LineTab)
   PointParams pp;
   int flags;
 };
@@ -122,100 +126,40 @@ struct PencilArgs {
 template <typename T, int N, bool DCT, int TKV = 0>
 struct PencilOps {
   using Cfg = PencilCfg<T, N, DCT, TKV>;
-  static constexpr int E = Cfg::E, G = Cfg::G, TK = Cfg::TK, LS = Cfg::LS, FP = Cfg::FP, RL = Cfg::RL;
+  using I = LineIdx<N>;
+  using F = LineFFT<T, N>;
+  static constexpr int E = Cfg::E, TK = Cfg::TK, FP = Cfg::FP;
+  using X = TileExchange<T, TK>;
+  using Tab = ColTables<T, N>;
 
-  // the TK lines of a tile are consecutive in memory (f0 and TK even: 16-byte pairs)
-  static constexpr bool PAIRS = pair_io<T>() && TK % 2 == 0;
-  static __device__ __forceinline__ int elem(int e) { return tile_elem<PAIRS>(threadIdx.x, Cfg::THREADS, e); }
+  // wavenumber index of B-side slot s: the cosine transforms keep the canonical
+  // pair order between their post- and pre-processing
+  static __device__ __forceinline__ int kx_of(int t, int s) { return DCT ? I::c_slot(t, s) : I::b_elem(t, s); }
 
-  // TK * N == THREADS * E: all E loads of a thread are issued before its stores
-  static __device__ __forceinline__ void load_tile(cplx<T>* buf, const cplx<T>* __restrict__ src, int f0) {
-    cplx<T> tmp[E];
+  // line (position f of every x-plane) between global memory and the A side
+  static __device__ __forceinline__ void load(cplx<T> (&v)[E], const cplx<T>* __restrict__ src, int t) {
 #pragma unroll
-    for (int e = 0; e < E; e += PAIRS ? 2 : 1) {
-      const int idx = elem(e);
-      const cplx<T>* p = &src[size_t(idx / TK) * FP + f0 + idx % TK];
-      if constexpr (PAIRS) ld_pair(p, tmp[e], tmp[e + 1]);
-      else tmp[e] = *p;
-    }
+    for (int s = 0; s < E; ++s) v[s] = src[size_t(real_pos<N, DCT>(I::a_elem(t, s))) * FP];
+  }
+  static __device__ __forceinline__ void store(const cplx<T> (&v)[E], cplx<T>* __restrict__ dst, int t) {
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int idx = elem(e);
-      buf[(idx % TK) * LS + pad(idx / TK)] = tmp[e];
+    for (int s = 0; s < E; ++s) dst[size_t(real_pos<N, DCT>(I::a_elem(t, s))) * FP] = v[s];
+  }
+  // forward x transform: A side -> spectrum at kx_of
+  static __device__ __forceinline__ void forward(cplx<T> (&v)[E], const X& x, int t, const Tab& tw, bool first_sync) {
+    F::forward(v, t, x, tw, first_sync);
+    if constexpr (DCT) {
+      F::canon(v, t);
+      F::dct2_post(v, t, tw);
     }
   }
-  static __device__ __forceinline__ void store_tile(const cplx<T>* buf, cplx<T>* __restrict__ dst, int f0) {
-#pragma unroll
-    for (int e = 0; e < E; e += PAIRS ? 2 : 1) {
-      const int idx = elem(e);
-      cplx<T>* p = &dst[size_t(idx / TK) * FP + f0 + idx % TK];
-      if constexpr (PAIRS) st_pair(p, buf[(idx % TK) * LS + pad(idx / TK)], buf[(idx % TK + 1) * LS + pad(idx / TK)]);
-      else *p = buf[(idx % TK) * LS + pad(idx / TK)];
+  // inverse x transform: spectrum at kx_of -> A side
+  static __device__ __forceinline__ void inverse(cplx<T> (&v)[E], const X& x, int t, const Tab& tw, bool first_sync) {
+    if constexpr (DCT) {
+      F::dct3_pre(v, t, tw);
+      F::uncanon(v, t);
     }
-  }
-
-  // forward x transform of the line; result in registers at kx = out_index<N,-1>
-  static __device__ __forceinline__ void forward(cplx<T> (&v)[E], cplx<T>* L, int t, const TwTables<T>& tw) {
-    if constexpr (!DCT) {
-      fft_line<T, N, -1>(v, L, t, tw.f, [&](int i) { return L[pad(i)]; });
-    } else {
-      fft_line<T, N, -1>(v, L, t, tw.f, [&](int i) { return L[pad(i < N / 2 ? 2 * i : 2 * (N - 1 - i) + 1)]; });
-      cplx<T> part[E];  // element (N - k) mod N of every slot
-      mirror_partners<T, N, RL>(v, part, t);
-#pragma unroll
-      for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-        for (int r = 0; r < RL; ++r) {
-          const int k = out_index<N, -1>(t, b, r);
-          cplx<T> w = tw.d[k];
-          v[b * RL + r] = cadd<T>(cmul<T>(v[b * RL + r], w), cmul<T>(part[b * RL + r], conjg<T>(w)));
-        }
-    }
-  }
-
-  // inverse x transform of register values at kx = out_index<N,-1>; result
-  // written to the line in natural x order (caller syncs before reading)
-  static __device__ __forceinline__ void inverse_to_line(cplx<T> (&v)[E], cplx<T>* L, int t,
-                                                         const TwTables<T>& tw) {
-    constexpr int RLI = radix_of<N, +1, Plan<N>::P - 1>();
-    if constexpr (!DCT) {
-      fft_regs<T, N, +1>(v, L, t, tw.i);
-      __syncwarp();
-#pragma unroll
-      for (int b = 0; b < E / RLI; ++b)
-#pragma unroll
-        for (int r = 0; r < RLI; ++r) L[pad(out_index<N, +1>(t, b, r))] = v[b * RLI + r];
-    } else {
-      // REDFT01 input exp(+i pi i/2N) (X[i] - i X[N-i]), X[N] = 0, formed in
-      // registers: the first inverse pass reads element i in the slot where
-      // the forward transform left element i
-      cplx<T> part[E];
-      mirror_partners<T, N, RL>(v, part, t);
-#pragma unroll
-      for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-        for (int r = 0; r < RL; ++r) {
-          const int i = out_index<N, -1>(t, b, r);
-          const cplx<T> a = v[b * RL + r];
-          cplx<T> u = a;
-          if (i != 0) {
-            const cplx<T> bb = part[b * RL + r];
-            u = mk<T>(a.x + bb.y, a.y - bb.x);
-          }
-          cplx<T> w = tw.d[i];
-          w.y = -w.y;
-          v[b * RL + r] = cmul<T>(u, w);
-        }
-      fft_regs<T, N, +1>(v, L, t, tw.i);
-      __syncwarp();
-#pragma unroll
-      for (int b = 0; b < E / RLI; ++b)
-#pragma unroll
-        for (int r = 0; r < RLI; ++r) {
-          const int n = out_index<N, +1>(t, b, r);
-          L[pad(n < N / 2 ? 2 * n : 2 * (N - 1 - n) + 1)] = v[b * RLI + r];
-        }
-    }
+    F::inverse(v, t, x, tw, first_sync);
   }
 };
 
@@ -241,27 +185,87 @@ __device__ __forceinline__ Mult<T> make_mult(T qx, T qy, T qz, T eps, const Poin
 __device__ __forceinline__ float rcp_rn(float x) { return __frcp_rn(x); }
 __device__ __forceinline__ double rcp_rn(double x) { return __drcp_rn(x); }
 
+// Both parts of a complex value as two independent reals (packed FP32x2)
+template <typename T>
+__device__ __forceinline__ cplx<T> both(T s) { return mk<T>(s, s); }
+template <typename T>
+__device__ __forceinline__ cplx<T> cfma(cplx<T> a, cplx<T> b, cplx<T> c) {
+  return mk<T>(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
+}
+template <typename T>
+__device__ __forceinline__ cplx<T> cmul2(cplx<T> a, cplx<T> b) { return mk<T>(a.x * b.x, a.y * b.y); }
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 1000 && !defined(SHB_NO_F32X2)
+template <>
+__device__ __forceinline__ float2 cfma<float>(float2 a, float2 b, float2 c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pk2(a)), "l"(pk2(b)), "l"(pk2(c)));
+  return upk2(r);
+}
+template <>
+__device__ __forceinline__ float2 cmul2<float>(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pk2(a)), "l"(pk2(b)));
+  return upk2(r);
+}
+#endif
+// products that no addition may absorb (ptxas fuses a packed mul and add)
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+// Reciprocals of the step's C2 (a normal number for every step that keeps psi
+// finite).  FP32: the hardware approximation and one Newton-Raphson iteration
+// r + r (1 - x r) in fused arithmetic; __frcp_rn, whose value it is for every
+// significand and the exponents from 2^-27 to 2^36 (checked over all of
+// them), carries a branch to a subnormal path in every use.
+__device__ __forceinline__ float rcp2(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return fmaf(r, fmaf(-x, r, 1.0f), r);
+}
+__device__ __forceinline__ float2 rcp2(float2 x) {
+  float2 r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(x.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(x.y));
+  const float2 e = cfma<float>(make_float2(-x.x, -x.y), r, make_float2(1.0f, 1.0f));
+  return cfma<float>(r, e, r);
+}
+// FP64: the 20-bit approximation and two iterations (relative error 2^-80 before
+// the last rounding)
+__device__ __forceinline__ double rcp2(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  r = fma(r, fma(-x, r, 1.0), r);
+  return fma(r, fma(-x, r, 1.0), r);
+}
+__device__ __forceinline__ double2 rcp2(double2 x) { return make_double2(rcp2(x.x), rcp2(x.y)); }
+
+// What bounds it: Neumann 256^3 FP32 moves 268 MB (41 us at the measured copy
+// rate) in 63 us; 22.4 M warp instructions (35 % of the issue slots), 2.2 M
+// shared-memory wavefronts; the waits are the HBM latency of the line loads and of
+// W.  The 16-values-per-thread form it replaces staged tiles in shared memory and
+// paired k with N - k by shuffles: 42 M instructions, 7.5 M wavefronts, 76 us.
+// Step pencil pass, before -> now: periodic 256^3 FP32 64.8 -> 57.3, Neumann 256^3
+// FP64 153 -> 137, Neumann 512^3 FP64 1672 -> 1180, periodic 512^3 FP32 637 -> 469,
+// periodic 128^3 FP64 23.1 -> 16.8, 64 x 64^3 FP32 68.7 -> 52.8 periodic, 83.3 -> 57.0
+// Neumann, FP64 update (kPencilStepU64) Neumann 256^3 95 -> 79 us.
 template <typename T, int N, bool DCT, int MODE, int TKV = 0>
 __global__ void __launch_bounds__(PencilCfg<T, N, DCT, TKV>::THREADS, PencilCfg<T, N, DCT, TKV>::min_blocks(MODE))
-pencil_kernel(PencilArgs<T> a) {
+pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
   using Cfg = PencilCfg<T, N, DCT, TKV>;
   using Ops = PencilOps<T, N, DCT, TKV>;
-  constexpr int E = Cfg::E, G = Cfg::G, TK = Cfg::TK, LS = Cfg::LS, FP = Cfg::FP, RL = Cfg::RL;
+  constexpr int E = Cfg::E, TK = Cfg::TK, FP = Cfg::FP, WB = Cfg::WB;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<T>* buf = reinterpret_cast<cplx<T>*>(smem_raw);
   double* scratch = reinterpret_cast<double*>(smem_raw + Cfg::red_off(MODE));
-  const TwTables<T> tw =
-      stage_twiddles<T, N>(reinterpret_cast<cplx<T>*>(smem_raw + Cfg::tw_off(MODE)), a.tw, threadIdx.x, Cfg::THREADS, DCT);
-  __syncthreads();  // every staged entry is written before any thread's first transform (kPencilAdjOut starts with one)
-  grid_dependency_wait();
 
   const int f0 = blockIdx.x * TK;
   const int rep = blockIdx.y;
-  const int line = threadIdx.x / G, t = threadIdx.x % G;
-  const int f = f0 + line;
-  cplx<T>* L = buf + line * LS;
-  const size_t plane_base = size_t(rep) * N * FP;
-  cplx<T>* wrow = a.w + (size_t(rep) * FP + f) * N;
+  const int c = threadIdx.x % TK, t = threadIdx.x / TK;
+  const int f = f0 + c;
+  const typename Ops::X x{buf + c};
+  const typename Ops::Tab tw(a.lt, t);
+  // this thread's slots of a spectrum kept aside: conflict-free, private
+  cplx<T>* aside = buf + size_t(TK) * N + threadIdx.x;
+  const size_t line = size_t(rep) * N * FP + f;  // position f of plane 0 (and of kx = 0)
   const T eps = T(a.pp.eps[rep]);
   const T scale = T(a.pp.scale);
 
@@ -280,28 +284,100 @@ pencil_kernel(PencilArgs<T> a) {
   const T qy = __ldg(&a.q[ky]);
   const T qz0 = __ldg(&a.q[kz]);
   const T qz1 = DCT ? __ldg(&a.q[kz + 1]) : T(0);
+  const T* qs = a.qs + t * E;
 
   cplx<T> v[E];
   KahanSum acc;
   const bool want_energy = (a.flags & kFlEnergy) != 0;
+  grid_dependency_wait();
 
-  if constexpr (MODE == kPencilStep || MODE == kPencilStepU64 || MODE == kPencilStepAdv) {
-    // this CTA's rows of W (TK x N complex, contiguous) are read after the forward
-    // transform: start bringing them into L2 now
-    if (threadIdx.x == 0)
-      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.w + (size_t(rep) * FP + f0) * N),
-                   "r"(uint32_t(size_t(TK) * N * sizeof(cplx<T>)))
-                   : "memory");
-    Ops::load_tile(buf, a.src + plane_base, f0);
-    __syncthreads();
-    Ops::forward(v, L, t, tw);
-    // the state W of this line, loaded after the transform: holding it through
-    // the transform costs the registers of a third resident CTA
-    cplx<T> wreg[E];
+  if constexpr (MODE == kPencilStep || MODE == kPencilStepU64) {
+    // CNAB2 and nothing else: this kernel is bound by the instructions it issues
+    // and fetches, so what only some runs ask for (kPencilStepGen) stays out of it
+    cplx<T>* w = a.w + line;
+    Ops::load(v, a.src + line, t);
+    // W is read after the transform: bring its rows (one 128-byte segment per
+    // kx) into L2 meanwhile.  Neumann 256^3 FP32: pencil pass 68.7 -> 64.3 us.
+    // Not for FP64 (137 -> 142 us), nor where the fields live in L2 anyway.
+    if constexpr (sizeof(T) == 4 && N >= 256) {
+      const cplx<T>* wt = a.w + size_t(rep) * N * FP + f0;
+      for (int k = threadIdx.x; k < N; k += Cfg::THREADS)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(wt + size_t(k) * FP));
+    }
+    Ops::forward(v, x, t, tw, false);
+    const T q02 = T(a.pp.q0 * a.pp.q0), alpha = T(a.pp.alpha);
+    const T h = T(0.5 * a.pp.dt), h3 = T(1.5 * a.pp.dt);
+    const T qyz0 = qy * qy + qz0 * qz0 - q02;
+    const cplx<T> qyz = mk<T>(qyz0, DCT ? qy * qy + qz1 * qz1 - q02 : qyz0);
+    double hd = 0.0, epsd = 0.0, qyz0d = 0.0, qyz1d = 0.0;
+    if constexpr (MODE == kPencilStepU64) {
+      hd = 0.5 * a.pp.dt;
+      epsd = a.pp.eps[rep];
+      const double qyd = __ldg(&a.qd[ky]), qz0d = __ldg(&a.qd[kz]);
+      qyz0d = qyd * qyd + qz0d * qz0d - a.pp.q0 * a.pp.q0;
+      if constexpr (DCT) {
+        const double qz1d = __ldg(&a.qd[kz + 1]);
+        qyz1d = qyd * qyd + qz1d * qz1d - a.pp.q0 * a.pp.q0;
+      }
+    }
+    cplx<T> finite = mk<T>(T(0), T(0));  // stays 0 unless a new coefficient is NaN / Inf
 #pragma unroll
-    for (int b = 0; b < E / RL; ++b)
+    for (int s0 = 0; s0 < E; s0 += WB) {
+      cplx<T> wreg[WB];
 #pragma unroll
-      for (int r = 0; r < RL; ++r) wreg[b * RL + r] = wrow[out_index<N, -1>(t, b, r)];
+      for (int i = 0; i < WB; ++i) wreg[i] = w[size_t(Ops::kx_of(t, s0 + i)) * FP];
+#pragma unroll
+      for (int i = 0; i < WB; ++i) {
+        const int s = s0 + i;
+        const cplx<T> nh = v[s];
+        cplx<T> wv = wreg[i];
+        cplx<T> pn;
+        if constexpr (MODE == kPencilStepU64) {
+          // FP32 fields with the per-mode multipliers and the update in FP64 from
+          // the FP64 wavenumbers, one rounding of each stored result.  A multiplier
+          // rounded to FP32 repeats the same relative error every step, which
+          // drifts a mode's amplitude linearly with the step count.
+          const double qxd = __ldg(&a.qds[t * E + s]);
+          auto update = [&](double qyzd, T n, T& w1, T& p1) {
+            const double e = qxd * qxd + qyzd;
+            const double hb = hd * (epsd - a.pp.alpha * e * e);
+            p1 = T((double(w1) + 3.0 * hd * double(n)) * rcp2(1.0 - hb));
+            w1 = T((1.0 + hb) * double(p1) - hd * double(n));
+          };
+          if constexpr (DCT) {
+            update(qyz0d, nh.x, wv.x, pn.x);
+            update(qyz1d, nh.y, wv.y, pn.y);
+          } else {
+            const double e = qxd * qxd + qyz0d;
+            const double hb = hd * (epsd - a.pp.alpha * e * e), i0 = rcp2(1.0 - hb);
+            pn.x = T((double(wv.x) + 3.0 * hd * double(nh.x)) * i0);
+            pn.y = T((double(wv.y) + 3.0 * hd * double(nh.y)) * i0);
+            wv.x = T((1.0 + hb) * double(pn.x) - hd * double(nh.x));
+            wv.y = T((1.0 + hb) * double(pn.y) - hd * double(nh.y));
+          }
+        } else {
+          const T qx = __ldg(&qs[s]);
+          // .x, .y: kz and kz + 1 (Neumann); one multiplier for both parts (periodic)
+          const cplx<T> d = cfma<T>(both<T>(qx), both<T>(qx), qyz);
+          const cplx<T> al = cfma<T>(cmul2<T>(both<T>(-alpha), d), d, both<T>(eps));
+          const cplx<T> ha = mk<T>(mul_rn(h, al.x), mul_rn(h, al.y));
+          const cplx<T> c2 = csub<T>(both<T>(T(1)), ha), c1 = cadd<T>(both<T>(T(1)), ha);
+          cplx<T> inv;
+          if constexpr (DCT) inv = rcp2(c2);
+          else inv = both<T>(rcp2(c2.x));
+          pn = cmul2<T>(cfma<T>(both<T>(h3), nh, wv), inv);
+          wv = cfma<T>(c1, pn, cmul2<T>(both<T>(-h), nh));
+        }
+        finite = cfma<T>(pn, both<T>(T(0)), finite);
+        w[size_t(Ops::kx_of(t, s)) * FP] = wv;
+        v[s] = cscale<T>(pn, scale);
+      }
+    }
+    if (!(finite.x == T(0) && finite.y == T(0))) *a.nonfinite = 1;
+  } else if constexpr (MODE == kPencilStepGen || MODE == kPencilStepU64Gen || MODE == kPencilStepAdv) {
+    cplx<T>* w = a.w + line;
+    Ops::load(v, a.src + line, t);
+    Ops::forward(v, x, t, tw, false);
     // mode-independent constants of the update; the (ky, kz) part of |q|^2 is
     // fixed for the line
     const T q02 = T(a.pp.q0 * a.pp.q0), alpha = T(a.pp.alpha);
@@ -312,7 +388,7 @@ pencil_kernel(PencilArgs<T> a) {
     // FP64 values of the FP32 update (see below); the scalars stay kernel parameters
     const double epsd = a.pp.eps[rep];
     double qyz0d = 0.0, qyz1d = 0.0;
-    if constexpr (MODE == kPencilStepU64 && sizeof(T) == 4) {
+    if constexpr (MODE == kPencilStepU64Gen) {
       const double qyd = __ldg(&a.qd[ky]), qz0d = __ldg(&a.qd[kz]);
       qyz0d = qyd * qyd + qz0d * qz0d - a.pp.q0 * a.pp.q0;
       if constexpr (DCT) {
@@ -321,27 +397,31 @@ pencil_kernel(PencilArgs<T> a) {
       }
     }
     bool bad = false;
+    // the state W of this line, read after the transform in batches of WB
+    // values: holding all of it through the transform costs the registers of
+    // the resident CTAs
 #pragma unroll
-    for (int b = 0; b < E / RL; ++b)
+    for (int s0 = 0; s0 < E; s0 += WB) {
+      cplx<T> wreg[WB];
 #pragma unroll
-      for (int r = 0; r < RL; ++r) {
-        const int kx = out_index<N, -1>(t, b, r);
-        const T qx = __ldg(&a.q[kx]);
+      for (int i = 0; i < WB; ++i) wreg[i] = w[size_t(Ops::kx_of(t, s0 + i)) * FP];
+#pragma unroll
+      for (int i = 0; i < WB; ++i) {
+        const int s = s0 + i;
+        const int kx = Ops::kx_of(t, s);
+        const T qx = __ldg(&qs[s]);
         const T qx2 = qx * qx;
-        cplx<T> wv = wreg[b * RL + r];
-        const cplx<T> nh = v[b * RL + r];
+        cplx<T> wv = wreg[i];
+        const cplx<T> nh = v[s];
         cplx<T> pn;
         // psihat^{n+1} = (W + 3dt/2 Nhat) / C2,  W' = C1 psihat^{n+1} - dt/2 Nhat  (CNAB2)
         // psihat^{n+1} = (psihat + dt Nhat) / (1 - dt aLin),  W' = psihat^{n+1} (IMEX Euler)
         const T d0 = qx2 + qyz0;
         const T a0 = eps - alpha * d0 * d0;
-        if constexpr (MODE == kPencilStepU64 && sizeof(T) == 4) {
-          // FP32 fields with the per-mode multipliers and the update in FP64 from
-          // the FP64 wavenumbers, one rounding of each stored result.  A multiplier
-          // rounded to FP32 repeats the same relative error every step, which
-          // drifts a mode's amplitude linearly with the step count.
+        if constexpr (MODE == kPencilStepU64Gen) {
+          // as kPencilStepU64
           const double hd = 0.5 * a.pp.dt;
-          const double qxd = __ldg(&a.qd[kx]);
+          const double qxd = __ldg(&a.qds[t * E + s]);
           const double e0 = qxd * qxd + qyz0d;
           const double b0 = epsd - a.pp.alpha * e0 * e0;
           if (cnab2) {
@@ -405,10 +485,11 @@ pencil_kernel(PencilArgs<T> a) {
           }
         }
         bad |= !isfinite(pn.x) || !isfinite(pn.y);
-        if (a.flags & kFlSpecOut) a.spec_out[(size_t(rep) * FP + f) * N + kx] = pn;
-        wrow[kx] = wv;
-        v[b * RL + r] = cscale<T>(pn, scale);
+        if (a.flags & kFlSpecOut) a.spec_out[line + size_t(kx) * FP] = pn;
+        w[size_t(kx) * FP] = wv;
+        v[s] = cscale<T>(pn, scale);
       }
+    }
     if (bad) *a.nonfinite = 1;
   } else if constexpr (MODE == kPencilEnergy) {
     // gradient part of the energy of the current state from its partial P,
@@ -417,73 +498,60 @@ pencil_kernel(PencilArgs<T> a) {
     const bool want_shell = (a.flags & kFlShell) != 0;
     if (want_shell)
       for (int i = threadIdx.x; i < Cfg::NSHELL; i += Cfg::THREADS) hist[i] = 0.0;
-    Ops::load_tile(buf, a.src + plane_base, f0);
+    Ops::load(v, a.src + line, t);
     __syncthreads();
-    Ops::forward(v, L, t, tw);
+    Ops::forward(v, x, t, tw, false);
     // P = IDFT_x(scale psihat): its forward x transform is N scale psihat
     // (REDFT10 after REDFT01: 2N scale psihat)
     const double inv = 1.0 / (a.pp.scale * (DCT ? 2 * N : N));
 #pragma unroll
-    for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-      for (int r = 0; r < RL; ++r) {
-        const int kx = out_index<N, -1>(t, b, r);
-        const T qx = __ldg(&a.q[kx]);
-        const double px = double(v[b * RL + r].x) * inv, py = double(v[b * RL + r].y) * inv;
-        const double q02 = double(a.pp.q0) * a.pp.q0;
+    for (int s = 0; s < E; ++s) {
+      const int kx = Ops::kx_of(t, s);
+      const T qx = __ldg(&qs[s]);
+      const double px = double(v[s].x) * inv, py = double(v[s].y) * inv;
+      const double q02 = double(a.pp.q0) * a.pp.q0;
+      if constexpr (!DCT) {
+        const double d = q02 - double(qx * qx + qy * qy + qz0 * qz0);
+        const double wgt = (kz == 0 || kz == N / 2) ? 1.0 : 2.0;
+        acc.add(wgt * d * d * (px * px + py * py));
+      } else {
+        const double wxy = (kx == 0 ? 0.5 : 1.0) * (ky == 0 ? 0.5 : 1.0);
+        const double d0 = q02 - double(qx * qx + qy * qy + qz0 * qz0);
+        const double d1 = q02 - double(qx * qx + qy * qy + qz1 * qz1);
+        acc.add(wxy * ((kz == 0 ? 0.5 : 1.0) * d0 * d0 * px * px + d1 * d1 * py * py));
+      }
+      if (want_shell) {
+        // shell = rint |(ix, iy, iz)|: signed indices (Nyquist +N/2) on the periodic
+        // grid, where every kz in (0, N/2) also stands for its conjugate
         if constexpr (!DCT) {
-          const double d = q02 - double(qx * qx + qy * qy + qz0 * qz0);
+          const int ix = kx <= N / 2 ? kx : kx - N, iy = ky <= N / 2 ? ky : ky - N;
+          const int sh = __double2int_rn(sqrt(double(ix * ix + iy * iy + kz * kz)));
           const double wgt = (kz == 0 || kz == N / 2) ? 1.0 : 2.0;
-          acc.add(wgt * d * d * (px * px + py * py));
+          atomicAdd(&hist[sh], wgt * (px * px + py * py));
         } else {
           const double wxy = (kx == 0 ? 0.5 : 1.0) * (ky == 0 ? 0.5 : 1.0);
-          const double d0 = q02 - double(qx * qx + qy * qy + qz0 * qz0);
-          const double d1 = q02 - double(qx * qx + qy * qy + qz1 * qz1);
-          acc.add(wxy * ((kz == 0 ? 0.5 : 1.0) * d0 * d0 * px * px + d1 * d1 * py * py));
-        }
-        if (want_shell) {
-          // shell = rint |(ix, iy, iz)|: signed indices (Nyquist +N/2) on the periodic
-          // grid, where every kz in (0, N/2) also stands for its conjugate
-          if constexpr (!DCT) {
-            const int ix = kx <= N / 2 ? kx : kx - N, iy = ky <= N / 2 ? ky : ky - N;
-            const int sh = __double2int_rn(sqrt(double(ix * ix + iy * iy + kz * kz)));
-            const double wgt = (kz == 0 || kz == N / 2) ? 1.0 : 2.0;
-            atomicAdd(&hist[sh], wgt * (px * px + py * py));
-          } else {
-            const double wxy = (kx == 0 ? 0.5 : 1.0) * (ky == 0 ? 0.5 : 1.0);
-            const int r2 = kx * kx + ky * ky;
-            const int s0 = __double2int_rn(sqrt(double(r2 + kz * kz)));
-            const int s1 = __double2int_rn(sqrt(double(r2 + (kz + 1) * (kz + 1))));
-            atomicAdd(&hist[s0], wxy * (kz == 0 ? 0.5 : 1.0) * px * px);
-            atomicAdd(&hist[s1], wxy * py * py);
-          }
+          const int r2 = kx * kx + ky * ky;
+          const int s0 = __double2int_rn(sqrt(double(r2 + kz * kz)));
+          const int s1 = __double2int_rn(sqrt(double(r2 + (kz + 1) * (kz + 1))));
+          atomicAdd(&hist[s0], wxy * (kz == 0 ? 0.5 : 1.0) * px * px);
+          atomicAdd(&hist[s1], wxy * py * py);
         }
       }
+    }
     if (want_shell) {
       __syncthreads();
       for (int i = threadIdx.x; i < Cfg::NSHELL; i += Cfg::THREADS)
         if (hist[i] != 0.0) atomicAdd(&a.shell[size_t(rep) * Cfg::NSHELL + i], hist[i]);
     }
-  } else if constexpr (MODE == kPencilSpec || MODE == kPencilAdjInit || MODE == kPencilAdj) {
-    Ops::load_tile(buf, a.src + plane_base, f0);
-    cplx<T> lreg[E];
-    if constexpr (MODE == kPencilAdj) {
+  } else if constexpr (MODE == kPencilSpec) {
+    Ops::load(v, a.src + line, t);
+    Ops::forward(v, x, t, tw, false);
+    // P = IDFT_x(scale psihat): its forward x transform is N scale psihat
+    const T inv = T(1.0 / (a.pp.scale * N));
 #pragma unroll
-      for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-        for (int r = 0; r < RL; ++r) lreg[b * RL + r] = wrow[out_index<N, -1>(t, b, r)];
-    }
-    __syncthreads();
-    Ops::forward(v, L, t, tw);
-    if constexpr (MODE == kPencilSpec) {
-      // P = IDFT_x(scale psihat): its forward x transform is N scale psihat
-      const T inv = T(1.0 / (a.pp.scale * N));
-#pragma unroll
-      for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-        for (int r = 0; r < RL; ++r)
-          a.spec_out[(size_t(rep) * FP + f) * N + out_index<N, -1>(t, b, r)] = cscale<T>(v[b * RL + r], inv);
-    } else if constexpr (!DCT) {
+    for (int s = 0; s < E; ++s) a.spec_out[line + size_t(Ops::kx_of(t, s)) * FP] = cscale<T>(v[s], inv);
+  } else if constexpr (MODE == kPencilAdjInit || MODE == kPencilAdj) {
+    if constexpr (!DCT) {
       // Discrete adjoint of CNAB2 (reverse of psi^{n+1} = A psi^n + B (c_n N^n - N^{n-1}), c_0 = 2,
       // c_n = 3):
       //   lambdahat^n = A lambdahat^{n+1} + ghat^n,  mu^n = B lambda^n,
@@ -493,38 +561,51 @@ pencil_kernel(PencilArgs<T> a) {
       //   dL/dtheta = sum_n <lambda^{n+1}, dt/2 (psihat^n + psihat^{n+1}) / C2 da/dtheta>
       // are regrouped by psihat^m: step n adds <lambda^{n+1} + [n >= 1] lambda^n, D psihat^n>, and
       // the first reverse step (spec_b set) also <lambda^{n+1}, D psihat^{n+1}>.
+      Ops::load(v, a.src + line, t);
+      Ops::forward(v, x, t, tw, false);
+      cplx<T>* w = a.w + line;
       const T q02 = T(a.pp.q0 * a.pp.q0), alpha = T(a.pp.alpha), h = T(0.5 * a.pp.dt);
       const T qyz = qy * qy + qz0 * qz0;
       const double wgt = ((kz == 0 || kz == N / 2) ? 1.0 : 2.0) / (double(N) * N * N);
       const double dadq0 = 4.0 * a.pp.alpha * a.pp.q0;
       const T coef = T(a.coef);
       const bool lam_n = a.coef != 0.0;  // n >= 1
-      // a thread's 16 terms are summed plainly (FP64); the per-CTA and
+      // a thread's E terms are summed plainly (FP64); the per-CTA and
       // per-step totals are combined in a fixed order
       double ge = 0.0, gq = 0.0;
+      constexpr int AB = WB / 2;
 #pragma unroll
-      for (int b = 0; b < E / RL; ++b)
+      for (int s0 = 0; s0 < E; s0 += AB) {
+        cplx<T> lreg[AB], preg[AB];
+        if constexpr (MODE == kPencilAdj) {
 #pragma unroll
-        for (int r = 0; r < RL; ++r) {
-          const int kx = out_index<N, -1>(t, b, r);
-          const T qx = __ldg(&a.q[kx]);
+          for (int i = 0; i < AB; ++i) {
+            const size_t k = size_t(Ops::kx_of(t, s0 + i)) * FP;
+            lreg[i] = w[k];
+            preg[i] = a.spec_a[line + k];
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < AB; ++i) {
+          const int s = s0 + i;
+          const size_t k = size_t(Ops::kx_of(t, s)) * FP;
+          const T qx = __ldg(&qs[s]);
           const T mq2 = qx * qx + qyz;
           const T d = mq2 - q02;
           const T al = eps - alpha * d * d;
           const T inv2 = rcp_rn(T(1) - h * al);
           const T am = (T(1) + h * al) * inv2, bm = h * inv2;
-          cplx<T> lam = v[b * RL + r];
+          cplx<T> lam = v[s];
           cplx<T> lnext = mk<T>(T(0), T(0));
           if constexpr (MODE == kPencilAdj) {
-            const cplx<T> l1 = lreg[b * RL + r];
+            const cplx<T> l1 = lreg[i];
             lam = mk<T>(am * l1.x + lam.x, am * l1.y + lam.y);
-            const size_t sidx = (size_t(rep) * FP + f) * N + kx;
-            const cplx<T> pa = a.spec_a[sidx];
+            const cplx<T> pa = preg[i];
             const double wx = double(l1.x) + (lam_n ? double(lam.x) : 0.0);
             const double wy = double(l1.y) + (lam_n ? double(lam.y) : 0.0);
             double dot = wx * double(pa.x) + wy * double(pa.y);
             if (a.spec_b) {
-              const cplx<T> pb = a.spec_b[sidx];
+              const cplx<T> pb = a.spec_b[line + k];
               dot += double(l1.x) * double(pb.x) + double(l1.y) * double(pb.y);
             }
             const double inner = wgt * double(bm) * dot;  // bm = dt/2 / C2
@@ -532,9 +613,10 @@ pencil_kernel(PencilArgs<T> a) {
             gq += inner * double(d);
             lnext = l1;
           }
-          wrow[kx] = lam;
-          v[b * RL + r] = cscale<T>(mk<T>(coef * lam.x - lnext.x, coef * lam.y - lnext.y), scale * bm);
+          w[k] = lam;
+          v[s] = cscale<T>(mk<T>(coef * lam.x - lnext.x, coef * lam.y - lnext.y), scale * bm);
         }
+      }
       if constexpr (MODE == kPencilAdj) {
         // each CTA accumulates into its own slot over the reverse sweep (fixed order)
         const double te = block_sum(ge, scratch);
@@ -548,53 +630,61 @@ pencil_kernel(PencilArgs<T> a) {
     }
   } else if constexpr (MODE == kPencilAdjOut) {
 #pragma unroll
-    for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-      for (int r = 0; r < RL; ++r) v[b * RL + r] = cscale<T>(wrow[out_index<N, -1>(t, b, r)], scale);
+    for (int s = 0; s < E; ++s) v[s] = cscale<T>(a.w[line + size_t(Ops::kx_of(t, s)) * FP], scale);
   } else if constexpr (MODE == kPencilXMul) {
-    Ops::load_tile(buf, a.src + plane_base, f0);
-    __syncthreads();
-    Ops::forward(v, L, t, tw);
+    Ops::load(v, a.src + line, t);
+    Ops::forward(v, x, t, tw, false);
     // P is the x-inverse of (scale X); its forward x transform is N scale X
     // (2N scale X for REDFT10 after REDFT01): multiply by m(q) / N (/ 2N)
     const T invn = T(1) / T(DCT ? 2 * N : N);
     const T q02 = T(a.pp.q0 * a.pp.q0), alpha = T(a.pp.alpha);
-    if constexpr (DCT) {
-      if (a.xmul == kXSinDx) {
-        // RODFT01(X)[x] = (-1)^x REDFT01(X reversed)[x] (the sine series of
-        // d/dx): slot kx takes -q_{N-kx} times coefficient N - kx, the mirror
-        // partner of kx; the plane pass applies (-1)^x
-        cplx<T> part[E];
-        mirror_partners<T, N, RL>(v, part, t);
+    if (DCT && a.xmul == kXSinDx) {
+      // RODFT01(X)[x] = (-1)^x REDFT01(X reversed)[x] (the sine series of
+      // d/dx): slot kx takes -q_{N-kx} times coefficient N - kx, the mirror of
+      // kx; the plane pass applies (-1)^x
+      using I = LineIdx<N>;
 #pragma unroll
-        for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-          for (int r = 0; r < RL; ++r) {
-            const int kx = out_index<N, -1>(t, b, r);
-            const T w = kx == 0 ? T(0) : -__ldg(&a.q[N - kx]) * invn;
-            v[b * RL + r] = cscale<T>(part[b * RL + r], w);
-          }
+      for (int r = 0; r < E / 2; ++r) {
+        const int k = I::c_elem(t, r), m = E - 1 - r;
+        const bool self = r == 0 && t == 0;  // the pair (0, N/2): each its own mirror
+        const cplx<T> lo = v[r], hi = v[m];
+        const T wk = k == 0 ? T(0) : -__ldg(&a.q[N - k]) * invn;
+        const T wm = self ? -__ldg(&a.q[N / 2]) * invn : -__ldg(&a.q[k]) * invn;
+        v[r] = cscale<T>(hi, wk);
+        v[m] = self ? cscale<T>(hi, wm) : cscale<T>(lo, wm);
       }
-    }
+    } else {
 #pragma unroll
-    for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-      for (int r = 0; r < RL; ++r) {
-        const T qx = __ldg(&a.q[out_index<N, -1>(t, b, r)]);
-        const cplx<T> val = v[b * RL + r];
-        if (a.xmul == kXSinDx) {
-          // done above
-        } else if (a.xmul == kXIqx) {
-          v[b * RL + r] = mk<T>(-qx * invn * val.y, qx * invn * val.x);
+      for (int s = 0; s < E; ++s) {
+        const T qx = __ldg(&qs[s]);
+        const cplx<T> val = v[s];
+        if (a.xmul == kXIqx) {
+          v[s] = mk<T>(-qx * invn * val.y, qx * invn * val.x);
         } else if (a.xmul == kXNegQx2) {
-          v[b * RL + r] = cscale<T>(val, -qx * qx * invn);
+          v[s] = cscale<T>(val, -qx * qx * invn);
         } else {
           const T d0 = qx * qx + qy * qy + qz0 * qz0 - q02;
           const T d1 = DCT ? qx * qx + qy * qy + qz1 * qz1 - q02 : d0;
-          v[b * RL + r] = mk<T>(alpha * d0 * d0 * invn * val.x, alpha * d1 * d1 * invn * val.y);
+          v[s] = mk<T>(alpha * d0 * d0 * invn * val.x, alpha * d1 * d1 * invn * val.y);
         }
       }
+    }
   } else if constexpr (MODE == kPencilStokes) {
+    // The three stress components go forward one after the other; the first two
+    // spectra wait in shared memory, the projector runs in registers, and the
+    // three velocity components go back.
+    cplx<T>* keep[2] = {aside, aside + size_t(TK) * N};
+    constexpr int TH = Cfg::THREADS;
+#pragma unroll 1
+    for (int comp = 0; comp < 3; ++comp) {
+      Ops::load(v, a.s3[comp] + line, t);
+      Ops::forward(v, x, t, tw, comp > 0);
+      if (comp < 2) {
+#pragma unroll
+        for (int s = 0; s < E; ++s) keep[comp][s * TH] = v[s];
+      }
+    }
+    const T ce = T(1.0 / a.pp.eta_rho);
     if constexpr (DCT) {
       // Neumann box: the stress came in as the cosine-transform partial of
       // (-1)^(x+y+z) S, whose REDFT10 at index k is the RODFT10 of S at index
@@ -602,228 +692,133 @@ pencil_kernel(PencilArgs<T> a) {
       // sine-wavenumber projector u = CM1 (S - CM2 (Vs . S)) of morphSurfK.cpp:
       // 862-882, Vs(m) = pi (m+1)/L, reads Vs = pi (N-k)/L at index k; the
       // inverse REDFT01 then yields (-1)^(x+y+z) u, unsigned by the plane pass.
-      cplx<T>* set[3] = {buf, buf + TK * LS, buf + 2 * TK * LS};
-#pragma unroll
-      for (int c = 0; c < 3; ++c) Ops::load_tile(set[c], a.s3[c] + plane_base, f0);
-      __syncthreads();
-#pragma unroll 1
-      for (int c = 0; c < 3; ++c) {
-        cplx<T>* Lc = set[c] + line * LS;
-        Ops::forward(v, Lc, t, tw);
-        __syncwarp();
-#pragma unroll
-        for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-          for (int r = 0; r < RL; ++r) Lc[pad(out_index<N, -1>(t, b, r))] = v[b * RL + r];
-      }
-      __syncwarp();
       const T q1 = __ldg(&a.q[1]);  // pi / L
       const T sy = T(N - ky) * q1, sz0 = T(N - kz) * q1, sz1 = T(N - kz - 1) * q1;
-      const T ce = T(1.0 / a.pp.eta_rho);
 #pragma unroll
-      for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-        for (int r = 0; r < RL; ++r) {
-          const int kx = out_index<N, -1>(t, b, r);
-          const T sx = T(N - kx) * q1;
-          const int o = line * LS + pad(kx);
-          const cplx<T> px = set[0][o], py = set[1][o], pz = set[2][o];
-          // .x holds kz, .y holds kz + 1
-          const T m0 = sx * sx + sy * sy + sz0 * sz0, m1 = sx * sx + sy * sy + sz1 * sz1;
-          const T i0 = T(1) / m0, i1 = T(1) / m1;
-          const T c0 = scale * ce * i0, c1 = scale * ce * i1;
-          const T d0 = sx * px.x + sy * py.x + sz0 * pz.x;
-          const T d1 = sx * px.y + sy * py.y + sz1 * pz.y;
-          set[0][o] = mk<T>(c0 * (px.x - sx * i0 * d0), c1 * (px.y - sx * i1 * d1));
-          set[1][o] = mk<T>(c0 * (py.x - sy * i0 * d0), c1 * (py.y - sy * i1 * d1));
-          set[2][o] = mk<T>(c0 * (pz.x - sz0 * i0 * d0), c1 * (pz.y - sz1 * i1 * d1));
-        }
-#pragma unroll 1
-      for (int c = 0; c < 3; ++c) {
-        cplx<T>* Lc = set[c] + line * LS;
-        __syncwarp();
-#pragma unroll
-        for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-          for (int r = 0; r < RL; ++r) v[b * RL + r] = Lc[pad(out_index<N, -1>(t, b, r))];
-        Ops::inverse_to_line(v, Lc, t, tw);
+      for (int s = 0; s < E; ++s) {
+        const T sx = T(N - Ops::kx_of(t, s)) * q1;
+        const cplx<T> px = keep[0][s * TH], py = keep[1][s * TH], pz = v[s];
+        // .x holds kz, .y holds kz + 1
+        const T m0 = sx * sx + sy * sy + sz0 * sz0, m1 = sx * sx + sy * sy + sz1 * sz1;
+        const T i0 = T(1) / m0, i1 = T(1) / m1;
+        const T c0 = scale * ce * i0, c1 = scale * ce * i1;
+        const T d0 = sx * px.x + sy * py.x + sz0 * pz.x;
+        const T d1 = sx * px.y + sy * py.y + sz1 * pz.y;
+        keep[0][s * TH] = mk<T>(c0 * (px.x - sx * i0 * d0), c1 * (px.y - sx * i1 * d1));
+        keep[1][s * TH] = mk<T>(c0 * (py.x - sy * i0 * d0), c1 * (py.y - sy * i1 * d1));
+        v[s] = mk<T>(c0 * (pz.x - sz0 * i0 * d0), c1 * (pz.y - sz1 * i1 * d1));
       }
-      __syncthreads();
-#pragma unroll
-      for (int c = 0; c < 3; ++c) Ops::store_tile(set[c], a.u3[c] + plane_base, f0);
     } else {
       // S -> u = scale CM1 (S - CM2 (q.S)),  CM1 = 1/(rho eta |q|^2), CM2 = q/|q|^2, both 0 at q = 0
-      cplx<T>* set[3] = {buf, buf + TK * LS, buf + 2 * TK * LS};
 #pragma unroll
-      for (int c = 0; c < 3; ++c) Ops::load_tile(set[c], a.s3[c] + plane_base, f0);
-      __syncthreads();
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        cplx<T>* Lc = set[c] + line * LS;
-        Ops::forward(v, Lc, t, tw);
-        __syncwarp();
-#pragma unroll
-        for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-          for (int r = 0; r < RL; ++r) Lc[pad(out_index<N, -1>(t, b, r))] = v[b * RL + r];
-      }
-      __syncwarp();
-      const T ce = T(1.0 / a.pp.eta_rho);
-#pragma unroll
-      for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-        for (int r = 0; r < RL; ++r) {
-          const int kx = out_index<N, -1>(t, b, r);
-          const T qx = __ldg(&a.q[kx]);
-          const T mq2 = qx * qx + qy * qy + qz0 * qz0;
-          const int o = line * LS + pad(kx);
-          const cplx<T> sx = set[0][o], sy = set[1][o], sz = set[2][o];
-          cplx<T> ux = mk<T>(T(0), T(0)), uy = ux, uz = ux;
-          if (mq2 != T(0)) {
-            const T inv = T(1) / mq2;
-            const T cm1 = scale * ce * inv;
-            const cplx<T> dot = mk<T>(qx * sx.x + qy * sy.x + qz0 * sz.x, qx * sx.y + qy * sy.y + qz0 * sz.y);
-            ux = mk<T>(cm1 * (sx.x - qx * inv * dot.x), cm1 * (sx.y - qx * inv * dot.y));
-            uy = mk<T>(cm1 * (sy.x - qy * inv * dot.x), cm1 * (sy.y - qy * inv * dot.y));
-            uz = mk<T>(cm1 * (sz.x - qz0 * inv * dot.x), cm1 * (sz.y - qz0 * inv * dot.y));
-          }
-          set[0][o] = ux;
-          set[1][o] = uy;
-          set[2][o] = uz;
+      for (int s = 0; s < E; ++s) {
+        const T qx = __ldg(&qs[s]);
+        const T mq2 = qx * qx + qy * qy + qz0 * qz0;
+        const cplx<T> sx = keep[0][s * TH], sy = keep[1][s * TH], sz = v[s];
+        cplx<T> ux = mk<T>(T(0), T(0)), uy = ux, uz = ux;
+        if (mq2 != T(0)) {
+          const T inv = T(1) / mq2;
+          const T cm1 = scale * ce * inv;
+          const cplx<T> dot = mk<T>(qx * sx.x + qy * sy.x + qz0 * sz.x, qx * sx.y + qy * sy.y + qz0 * sz.y);
+          ux = mk<T>(cm1 * (sx.x - qx * inv * dot.x), cm1 * (sx.y - qx * inv * dot.y));
+          uy = mk<T>(cm1 * (sy.x - qy * inv * dot.x), cm1 * (sy.y - qy * inv * dot.y));
+          uz = mk<T>(cm1 * (sz.x - qz0 * inv * dot.x), cm1 * (sz.y - qz0 * inv * dot.y));
         }
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        cplx<T>* Lc = set[c] + line * LS;
-        __syncwarp();
-#pragma unroll
-        for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-          for (int r = 0; r < RL; ++r) v[b * RL + r] = Lc[pad(out_index<N, -1>(t, b, r))];
-        Ops::inverse_to_line(v, Lc, t, tw);
+        keep[0][s * TH] = ux;
+        keep[1][s * TH] = uy;
+        v[s] = uz;
       }
-      __syncthreads();
+    }
+#pragma unroll 1
+    for (int comp = 2; comp >= 0; --comp) {
+      if (comp < 2) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) Ops::store_tile(set[c], a.u3[c] + plane_base, f0);
+        for (int s = 0; s < E; ++s) v[s] = keep[comp][s * TH];
+      }
+      Ops::inverse(v, x, t, tw, true);
+      Ops::store(v, a.u3[comp] + line, t);
     }
   } else {  // kPencilInit(Adv): W^0 from psi^0 and N(psi^0); P^0 from psi^0
-    Ops::load_tile(buf, a.src + plane_base, f0);
-    __syncthreads();
-    Ops::forward(v, L, t, tw);
-    cplx<T> vn[E];
-    __syncthreads();
-    Ops::load_tile(buf, a.src2 + plane_base, f0);
-    __syncthreads();
-    Ops::forward(vn, L, t, tw);
+    constexpr int TH = Cfg::THREADS;
+    Ops::load(v, a.src2 + line, t);
+    Ops::forward(v, x, t, tw, false);
 #pragma unroll
-    for (int b = 0; b < E / RL; ++b)
+    for (int s = 0; s < E; ++s) aside[s * TH] = v[s];
+    Ops::load(v, a.src + line, t);
+    Ops::forward(v, x, t, tw, true);
 #pragma unroll
-      for (int r = 0; r < RL; ++r) {
-        const int kx = out_index<N, -1>(t, b, r);
-        const T qx = __ldg(&a.q[kx]);
-        const cplx<T> ph = v[b * RL + r], nh = vn[b * RL + r];
-        cplx<T> wv;
-        const Mult<T> m0 = make_mult<T>(qx, qy, qz0, eps, a.pp);
-        const Mult<T> m1 = DCT ? make_mult<T>(qx, qy, qz1, eps, a.pp) : m0;
-        if (a.pp.scheme == kCNAB2) {
-          wv.x = m0.c1 * ph.x - T(0.5 * a.pp.dt) * nh.x;
-          wv.y = m1.c1 * ph.y - T(0.5 * a.pp.dt) * nh.y;
-        } else {
-          wv = ph;
-        }
-        wrow[kx] = wv;
-        v[b * RL + r] = cscale<T>(ph, scale);
+    for (int s = 0; s < E; ++s) {
+      const T qx = __ldg(&qs[s]);
+      const cplx<T> ph = v[s], nh = aside[s * TH];
+      cplx<T> wv;
+      const Mult<T> m0 = make_mult<T>(qx, qy, qz0, eps, a.pp);
+      const Mult<T> m1 = DCT ? make_mult<T>(qx, qy, qz1, eps, a.pp) : m0;
+      if (a.pp.scheme == kCNAB2) {
+        wv.x = m0.c1 * ph.x - T(0.5 * a.pp.dt) * nh.x;
+        wv.y = m1.c1 * ph.y - T(0.5 * a.pp.dt) * nh.y;
+      } else {
+        wv = ph;
       }
-  }
-
-  if constexpr (MODE == kPencilStep || MODE == kPencilStepU64 || MODE == kPencilInit || MODE == kPencilXMul ||
-                MODE == kPencilAdjInit ||
-                MODE == kPencilAdj || MODE == kPencilAdjOut) {
-    Ops::inverse_to_line(v, L, t, tw);
-    __syncthreads();
-    Ops::store_tile(buf, a.dst + plane_base, f0);
-  } else if constexpr (MODE == kPencilStepAdv || MODE == kPencilInitAdv) {
-    if constexpr (DCT) {
-      // v = scale psihat^{n+1}; emit the partials of v and, where asked, of
-      // -q_x^2 v (the x half of the substrate's in-plane Laplacian) and of
-      // opSH v (L psi of the Stokes stress, cosFFT/comet/morphSurfK.cpp:686-696),
-      // one inverse x transform each
-      cplx<T>* stash = buf + TK * LS + line * LS;
-      __syncwarp();
-#pragma unroll
-      for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-        for (int r = 0; r < RL; ++r) stash[pad(out_index<N, -1>(t, b, r))] = v[b * RL + r];
-      __syncwarp();
-      const T q02 = T(a.pp.q0 * a.pp.q0), alpha = T(a.pp.alpha);
-      cplx<T>* outs[3] = {a.dst, a.dst_x, a.dst_sh};
-#pragma unroll 1
-      for (int o = 0; o < 3; ++o) {
-        if (!outs[o]) continue;  // uniform over the CTA
-#pragma unroll
-        for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-          for (int r = 0; r < RL; ++r) {
-            const int kx = out_index<N, -1>(t, b, r);
-            const cplx<T> val = stash[pad(kx)];
-            const T qx = __ldg(&a.q[kx]);
-            if (o == 0) {
-              v[b * RL + r] = val;
-            } else if (o == 1) {
-              v[b * RL + r] = cscale<T>(val, -qx * qx);
-            } else {  // the pair holds kz and kz + 1
-              const T d0 = qx * qx + qy * qy + qz0 * qz0 - q02;
-              const T d1 = qx * qx + qy * qy + qz1 * qz1 - q02;
-              v[b * RL + r] = mk<T>(alpha * d0 * d0 * val.x, alpha * d1 * d1 * val.y);
-            }
-          }
-        Ops::inverse_to_line(v, L, t, tw);
-        __syncthreads();
-        Ops::store_tile(buf, outs[o] + plane_base, f0);
-        __syncthreads();
-      }
-    } else {
-      // v = scale psihat^{n+1}; emit the partials of v, i q_x v and opSH v
-      // (periodicFFT/pf3d.cpp:404-407), one inverse x transform each
-      cplx<T>* stash = buf + TK * LS + line * LS;
-      __syncwarp();
-#pragma unroll
-      for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-        for (int r = 0; r < RL; ++r) stash[pad(out_index<N, -1>(t, b, r))] = v[b * RL + r];
-      __syncwarp();
-      const T q02 = T(a.pp.q0 * a.pp.q0), alpha = T(a.pp.alpha);
-      cplx<T>* outs[3] = {a.dst, a.dst_x, a.dst_sh};
-#pragma unroll 1
-      for (int o = 0; o < 3; ++o) {
-#pragma unroll
-        for (int b = 0; b < E / RL; ++b)
-#pragma unroll
-          for (int r = 0; r < RL; ++r) {
-            const int kx = out_index<N, -1>(t, b, r);
-            const cplx<T> val = stash[pad(kx)];
-            const T qx = __ldg(&a.q[kx]);
-            if (o == 0) {
-              v[b * RL + r] = val;
-            } else if (o == 1) {
-              v[b * RL + r] = mk<T>(-qx * val.y, qx * val.x);
-            } else {
-              const T d = qx * qx + qy * qy + qz0 * qz0 - q02;
-              v[b * RL + r] = cscale<T>(val, alpha * d * d);
-            }
-          }
-        Ops::inverse_to_line(v, L, t, tw);
-        __syncthreads();
-        Ops::store_tile(buf, outs[o] + plane_base, f0);
-        __syncthreads();
-      }
+      a.w[line + size_t(Ops::kx_of(t, s)) * FP] = wv;
+      v[s] = cscale<T>(ph, scale);
     }
   }
 
-  if (want_energy && (MODE == kPencilStep || MODE == kPencilStepU64 || MODE == kPencilStepAdv ||
+  if constexpr (MODE == kPencilStep || MODE == kPencilStepGen || MODE == kPencilStepU64 || MODE == kPencilStepU64Gen || MODE == kPencilInit || MODE == kPencilXMul ||
+                MODE == kPencilAdjInit || MODE == kPencilAdj || MODE == kPencilAdjOut) {
+    Ops::inverse(v, x, t, tw, MODE != kPencilAdjOut);
+    Ops::store(v, a.dst + line, t);
+  } else if constexpr (MODE == kPencilStepAdv || MODE == kPencilInitAdv) {
+    // v = scale psihat^{n+1}; emit its partial, one inverse x transform each, and
+    //   periodic: those of i q_x v and opSH v (periodicFFT/pf3d.cpp:404-407)
+    //   Neumann, where asked: those of -q_x^2 v (the x half of the substrate's
+    //   in-plane Laplacian) and of opSH v (L psi of the Stokes stress,
+    //   cosFFT/comet/morphSurfK.cpp:686-696)
+    constexpr int TH = Cfg::THREADS;
+    const T q02 = T(a.pp.q0 * a.pp.q0), alpha = T(a.pp.alpha);
+#pragma unroll
+    for (int s = 0; s < E; ++s) aside[s * TH] = v[s];
+    cplx<T>* outs[3] = {a.dst, a.dst_x, a.dst_sh};
+#pragma unroll 1
+    for (int o = 0; o < 3; ++o) {
+      if (!outs[o]) continue;  // uniform over the grid
+      if (o > 0) {
+#pragma unroll
+        for (int s = 0; s < E; ++s) {
+          const cplx<T> val = aside[s * TH];
+          const T qx = __ldg(&qs[s]);
+          if (o == 1) {
+            v[s] = DCT ? cscale<T>(val, -qx * qx) : mk<T>(-qx * val.y, qx * val.x);
+          } else {  // Neumann: the pair holds kz and kz + 1
+            const T d0 = qx * qx + qy * qy + qz0 * qz0 - q02;
+            const T d1 = DCT ? qx * qx + qy * qy + qz1 * qz1 - q02 : d0;
+            v[s] = mk<T>(alpha * d0 * d0 * val.x, alpha * d1 * d1 * val.y);
+          }
+        }
+      }
+      Ops::inverse(v, x, t, tw, true);
+      Ops::store(v, outs[o] + line, t);
+    }
+  }
+
+  if (want_energy && (MODE == kPencilStepGen || MODE == kPencilStepU64Gen || MODE == kPencilStepAdv ||
                       MODE == kPencilEnergy)) {
     const double tot = block_sum(acc.s, scratch);
     if (threadIdx.x == 0) a.red[size_t(rep) * gridDim.x + blockIdx.x] = tot;
   }
+}
+
+// dst[rep][r][c] -> [rep][c][r] of complex values: the checkpoint file keeps W as
+// [f][kx], the device as [kx][f]
+template <typename T>
+__global__ void transpose_kernel(const cplx<T>* __restrict__ src, cplx<T>* __restrict__ dst, int rows, int cols) {
+  __shared__ cplx<T> tile[16][17];
+  const size_t base = size_t(blockIdx.z) * rows * cols;
+  const int c = blockIdx.x * 16 + threadIdx.x, r = blockIdx.y * 16 + threadIdx.y;
+  tile[threadIdx.y][threadIdx.x] = src[base + size_t(r) * cols + c];
+  __syncthreads();
+  const int c2 = blockIdx.x * 16 + threadIdx.y, r2 = blockIdx.y * 16 + threadIdx.x;
+  dst[base + size_t(c2) * rows + r2] = tile[threadIdx.x][threadIdx.y];
 }
 
 }  // namespace shb

@@ -47,7 +47,7 @@ enum PassFlags : int {
   kFlL1 = 2,        // plane: L1 monitor partial sums
   kFlEnergy = 4,    // plane / pencil: energy partial sums
   kFlRealOut = 8,   // plane step: write psi (T) to real_out
-  kFlSpecOut = 16,  // pencil step: write psihat^{n+1} (pencil-major) to spec_out
+  kFlSpecOut = 16,  // pencil step: write psihat^{n+1} to spec_out
   kFlShell = 32,    // pencil energy pass: spectral power per |k| shell into PencilArgs::shell
 };
 

@@ -61,6 +61,13 @@ __global__ void to_double_kernel(const T* __restrict__ src, double* __restrict__
 // lowest such shell on a tie)
 __global__ void shell_argmax_kernel(const double* shell, int nshell, double dq, double* out);
 
+// device memory of one call, freed when the call returns
+template <class P>
+struct DeviceScratch {
+  P* p = nullptr;
+  ~DeviceScratch() { cudaFree(p); }
+};
+
 struct SolverBase {
   sh_params p{};
   std::vector<double> eps;
@@ -158,6 +165,7 @@ struct Solver final : SolverBase {
   cplx<T>* P = nullptr;
   cplx<T>* Nt = nullptr;
   cplx<T>* tw = nullptr;  // [forward | inverse | quarter-wave] twiddle table
+  cplx<T>* lt = nullptr;  // line tables (LineTab)
   // Stokes advection (periodic): partials of i q_x psihat and opSH psihat, the
   // three stress / velocity partials, and the real fields
   // psi, d_x psi, d_y psi, d_z psi, L psi (then u_x), u_y, u_z
@@ -185,9 +193,9 @@ struct Solver final : SolverBase {
   // adjoint work buffers, kept for the handle's lifetime once allocated
   struct AdjBufs {
     cplx<T>* ck = nullptr;   // checkpoints: nseg states x {W, P, Nt}
-    cplx<T>* hs = nullptr;   // (k+1) psihat of a segment, pencil-major
+    cplx<T>* hs = nullptr;   // (k+1) psihat of a segment
     T* hr = nullptr;         // (k+1) psi of a segment
-    cplx<T>* lam = nullptr;  // lambdahat, pencil-major
+    cplx<T>* lam = nullptr;  // lambdahat [kx][f]
     cplx<T>* gp = nullptr;   // partial of g
     cplx<T>* mp = nullptr;   // partial of c_n mu^{n+1} - mu^{n+2}
     double* red = nullptr;   // per-CTA gradient sums of the reverse sweep
@@ -199,12 +207,14 @@ struct Solver final : SolverBase {
       cudaFree(red); cudaFree(acc); cudaFree(fin);
     }
   } adj;
-  // adjoint: per-step history of a recomputed segment (psihat pencil-major, psi real)
+  // adjoint: per-step history of a recomputed segment (psihat [kx][f], psi real)
   cplx<T>* hist_spec = nullptr;
   T* hist_real = nullptr;
   int hist_pos = 0;
   T* q = nullptr;
   double* qd = nullptr;  // the wavenumbers in FP64 (the FP32 spectral update uses them)
+  T* qs = nullptr;       // both in the slot order of the pencil pass
+  double* qds = nullptr;
 
   ~Solver() override {
     if (stream) cudaStreamSynchronize(stream);
@@ -212,8 +222,11 @@ struct Solver final : SolverBase {
     cudaFree(P);
     cudaFree(Nt);
     cudaFree(tw);
+    cudaFree(lt);
     cudaFree(q);
     cudaFree(qd);
+    cudaFree(qs);
+    cudaFree(qds);
     cudaFree(Px);
     cudaFree(PSH);
     for (auto* p3 : S3) cudaFree(p3);
@@ -263,7 +276,12 @@ struct Solver final : SolverBase {
   // the plain step's pencil pass: FP32 fields take their CNAB2 multipliers in
   // FP64 when the handle asks for it (SH_FP32_UPDATE64)
   int launch_pencil_step(const PencilArgs<T>& b, int reps = 0) {
-    if (sizeof(T) == 4 && p.precision == SH_FP32_UPDATE64) return launch_pencil<kPencilStepU64>(b, reps);
+    const bool gen = p.scheme != kCNAB2 || b.flags != 0;
+    if constexpr (sizeof(T) == 4) {
+      if (p.precision == SH_FP32_UPDATE64)
+        return gen ? launch_pencil<kPencilStepU64Gen>(b, reps) : launch_pencil<kPencilStepU64>(b, reps);
+    }
+    if (gen) return launch_pencil<kPencilStepGen>(b, reps);
     return launch_pencil<kPencilStep>(b, reps);
   }
 
@@ -276,8 +294,8 @@ struct Solver final : SolverBase {
 
   int setup() override {
     const size_t fe = field_elems();
-    if (p.advection && !QC::fits(kPencilStokes)) {
-      err = "Stokes advection is not built for this size and precision (its pencil pass does not fit a CTA)";
+    if (p.advection && N == 512 && sizeof(T) == 8 && DCT) {
+      err = "Stokes advection is not built for this size, precision and boundary";
       return SH_EUNSUPPORTED;
     }
     SHB_CUDA(dev_malloc(&W, fe * sizeof(cplx<T>)));
@@ -318,6 +336,9 @@ struct Solver final : SolverBase {
     SHB_CUDA(dev_malloc(&tw, tw_total<N>() * sizeof(cplx<T>)));
     SHB_CUDA(dev_malloc(&q, N * sizeof(T)));
     SHB_CUDA(dev_malloc(&qd, N * sizeof(double)));
+    SHB_CUDA(dev_malloc(&lt, LineTab<N>::total * sizeof(cplx<T>)));
+    SHB_CUDA(dev_malloc(&qs, N * sizeof(T)));
+    SHB_CUDA(dev_malloc(&qds, N * sizeof(double)));
     SHB_CUDA(dev_malloc(&d_red_plane, size_t(p.batch) * N * CL * 3 * sizeof(double)));
     SHB_CUDA(dev_malloc(&d_red_spec, size_t(p.batch) * QC::TILES * sizeof(double)));
     std::vector<cplx<T>> htw;
@@ -336,13 +357,30 @@ struct Solver final : SolverBase {
     SHB_CUDA(cudaMemcpy(qd, hqd.data(), N * sizeof(double), cudaMemcpyHostToDevice));
     SHB_CUDA(cudaMemcpy(tw, htw.data(), htw.size() * sizeof(cplx<T>), cudaMemcpyHostToDevice));
     SHB_CUDA(cudaMemcpy(q, hq.data(), N * sizeof(T), cudaMemcpyHostToDevice));
+    std::vector<cplx<T>> hlt;
+    host_line_tables<T, N>(hlt);
+    std::vector<T> hqs(N);
+    std::vector<double> hqds(N);
+    for (int t = 0; t < QC::G; ++t)
+      for (int s = 0; s < QC::E; ++s) {
+        const int k = DCT ? LineIdx<N>::c_slot(t, s) : LineIdx<N>::b_elem(t, s);
+        hqs[t * QC::E + s] = hq[k];
+        hqds[t * QC::E + s] = hqd[k];
+      }
+    SHB_CUDA(cudaMemcpy(lt, hlt.data(), hlt.size() * sizeof(cplx<T>), cudaMemcpyHostToDevice));
+    SHB_CUDA(cudaMemcpy(qs, hqs.data(), N * sizeof(T), cudaMemcpyHostToDevice));
+    SHB_CUDA(cudaMemcpy(qds, hqds.data(), N * sizeof(double), cudaMemcpyHostToDevice));
     int rc;
     if ((rc = set_attrs(plane_fn<kPlaneStep>(), PC::SMEM, true))) return rc;
     if ((rc = set_attrs(plane_fn<kPlaneInit>(), PC::SMEM, true))) return rc;
     if ((rc = set_attrs(plane_fn<kPlaneGetPsi>(), PC::SMEM, true))) return rc;
     if ((rc = set_attrs(plane_fn<kPlaneInvReal>(), PC::SMEM, true))) return rc;
     if ((rc = set_pencil_attrs<kPencilStep>())) return rc;
-    if ((rc = set_pencil_attrs<kPencilStepU64>())) return rc;
+    if constexpr (sizeof(T) == 4) {
+      if ((rc = set_pencil_attrs<kPencilStepU64>())) return rc;
+      if ((rc = set_pencil_attrs<kPencilStepU64Gen>())) return rc;
+    }
+    if ((rc = set_pencil_attrs<kPencilStepGen>())) return rc;
     if ((rc = set_pencil_attrs<kPencilInit>())) return rc;
     if ((rc = set_pencil_attrs<kPencilEnergy>())) return rc;
     if ((rc = set_pencil_attrs<kPencilStepAdv>())) return rc;
@@ -468,9 +506,11 @@ struct Solver final : SolverBase {
   }
   PencilArgs<T> pencil_args() const {
     PencilArgs<T> a{};
-    a.tw = tw;
+    a.lt = lt;
     a.q = q;
     a.qd = qd;
+    a.qs = qs;
+    a.qds = qds;
     a.pp = point_params();
     a.red = d_red_spec;
     a.nonfinite = d_flag;
@@ -914,7 +954,13 @@ struct Solver final : SolverBase {
   int save_state(void* host) override {
     const size_t fb = field_elems() * sizeof(cplx<T>);
     char* h = static_cast<char*>(host);
-    SHB_CUDA(cudaMemcpyAsync(h, W, fb, cudaMemcpyDeviceToHost, stream));
+    // the file keeps W as [f][kx]
+    DeviceScratch<cplx<T>> wt;
+    SHB_CUDA(dev_malloc(&wt.p, fb));
+    transpose_kernel<T><<<dim3(FP / 16, N / 16, p.batch), dim3(16, 16), 0, stream>>>(W, wt.p, N, FP);
+    SHB_CUDA(cudaGetLastError());
+    ++launches;
+    SHB_CUDA(cudaMemcpyAsync(h, wt.p, fb, cudaMemcpyDeviceToHost, stream));
     SHB_CUDA(cudaMemcpyAsync(h + fb, P, fb, cudaMemcpyDeviceToHost, stream));
     SHB_CUDA(cudaMemcpyAsync(h + 2 * fb, Nt, fb, cudaMemcpyDeviceToHost, stream));
     if (p.advection) {
@@ -928,7 +974,12 @@ struct Solver final : SolverBase {
     adj_end = -1;
     const size_t fb = field_elems() * sizeof(cplx<T>);
     const char* h = static_cast<const char*>(host);
-    SHB_CUDA(cudaMemcpyAsync(W, h, fb, cudaMemcpyHostToDevice, stream));
+    DeviceScratch<cplx<T>> wt;
+    SHB_CUDA(dev_malloc(&wt.p, fb));
+    SHB_CUDA(cudaMemcpyAsync(wt.p, h, fb, cudaMemcpyHostToDevice, stream));
+    transpose_kernel<T><<<dim3(N / 16, FP / 16, p.batch), dim3(16, 16), 0, stream>>>(wt.p, W, FP, N);
+    SHB_CUDA(cudaGetLastError());
+    ++launches;
     SHB_CUDA(cudaMemcpyAsync(P, h + fb, fb, cudaMemcpyHostToDevice, stream));
     SHB_CUDA(cudaMemcpyAsync(Nt, h + 2 * fb, fb, cudaMemcpyHostToDevice, stream));
     if (p.advection) {
@@ -1025,7 +1076,7 @@ struct Solver final : SolverBase {
       ADJ_CUDA(cudaMemcpyAsync(c + 2 * fe, Nt, fb, cudaMemcpyDeviceToDevice, stream));
       const int s1 = (sg + 1) * K < nsteps ? (sg + 1) * K : nsteps;
       if (sg == nseg - 1) {
-        // the last segment keeps its states (psihat^n pencil-major, psi^n real) as
+        // the last segment keeps its states (psihat^n [kx][f], psi^n real) as
         // the reverse sweep needs them, so the backward does not recompute it
         PencilArgs<T> b = pencil_args();
         b.src = P;
