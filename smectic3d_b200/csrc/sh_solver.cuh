@@ -1,6 +1,7 @@
 // Host-side solver: owns the device state of one handle and sequences the
 // plane and pencil passes of each time step.
 #pragma once
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -10,6 +11,7 @@
 #include "../../include/smectic_b200.h"
 #include "pencil_kernel.cuh"
 #include "plane_kernel.cuh"
+#include "split_kernel.cuh"
 #include "surface_kernel.cuh"
 
 namespace shb {
@@ -164,6 +166,10 @@ struct Solver final : SolverBase {
   cplx<T>* W = nullptr;
   cplx<T>* P = nullptr;
   cplx<T>* Nt = nullptr;
+  // work slab of the split plane pass (split_kernel.cuh), slab_planes x-planes;
+  // null where the plane pass is one kernel
+  cplx<T>* slab = nullptr;
+  int slab_planes = 0;
   cplx<T>* tw = nullptr;  // [forward | inverse | quarter-wave] twiddle table
   cplx<T>* lt = nullptr;  // line tables (LineTab)
   // Stokes advection (periodic): partials of i q_x psihat and opSH psihat, the
@@ -221,6 +227,7 @@ struct Solver final : SolverBase {
     cudaFree(W);
     cudaFree(P);
     cudaFree(Nt);
+    cudaFree(slab);
     cudaFree(tw);
     cudaFree(lt);
     cudaFree(q);
@@ -243,6 +250,12 @@ struct Solver final : SolverBase {
   }
 
   size_t field_elems() const { return size_t(p.batch) * N * FP; }
+
+  // planes too large for one CTA go through the split passes
+    static constexpr bool kSplit = N >= 256;
+  static constexpr size_t kSlabBytes = size_t(64) << 20;
+  using YC = YcolCfg<T, N, DCT>;
+  using ZC = ZrowCfg<T, N, DCT>;
 
   PointParams point_params() const {
     PointParams pp;
@@ -301,6 +314,16 @@ struct Solver final : SolverBase {
     SHB_CUDA(dev_malloc(&W, fe * sizeof(cplx<T>)));
     SHB_CUDA(dev_malloc(&P, fe * sizeof(cplx<T>)));
     SHB_CUDA(dev_malloc(&Nt, fe * sizeof(cplx<T>)));
+    if constexpr (kSplit) {
+      constexpr size_t plane_bytes = size_t(YC::SP) * sizeof(cplx<T>);
+      const long long planes = (long long)p.batch * N;
+      slab_planes = int(std::min<long long>(planes, std::max<long long>(1, kSlabBytes / plane_bytes)));
+      if (dev_malloc(&slab, slab_planes * plane_bytes) != cudaSuccess) {
+        // the fields themselves fit: keep the clustered plane pass, which needs no slab
+        cudaGetLastError();
+        slab = nullptr;
+      }
+    }
     if (p.advection) {
       // periodic: partials of psi, i q_x psi and opSH psi; Neumann: of psi and
       // opSH psi (its gradient is a difference stencil in real space)
@@ -339,7 +362,7 @@ struct Solver final : SolverBase {
     SHB_CUDA(dev_malloc(&lt, LineTab<N>::total * sizeof(cplx<T>)));
     SHB_CUDA(dev_malloc(&qs, N * sizeof(T)));
     SHB_CUDA(dev_malloc(&qds, N * sizeof(double)));
-    SHB_CUDA(dev_malloc(&d_red_plane, size_t(p.batch) * N * CL * 3 * sizeof(double)));
+    SHB_CUDA(dev_malloc(&d_red_plane, size_t(p.batch) * N * std::max(CL, kSplit ? ZC::BLOCKS : 1) * 3 * sizeof(double)));
     SHB_CUDA(dev_malloc(&d_red_spec, size_t(p.batch) * QC::TILES * sizeof(double)));
     std::vector<cplx<T>> htw;
     host_twiddles<T, N>(htw);
@@ -395,8 +418,73 @@ struct Solver final : SolverBase {
     if ((rc = set_attrs(plane_fn<kPlaneInvMulFwd>(), PC::SMEM, true))) return rc;
     if ((rc = set_attrs(plane_fn<kPlaneAdvN>(), PC::SMEM, true))) return rc;
     if ((rc = set_attrs(plane_fn<kPlaneMulFwd>(), PC::SMEM, true))) return rc;
+    if constexpr (kSplit) {
+      if ((rc = set_attrs(&ycol_kernel<T, N, DCT, true>, YC::SMEM, false))) return rc;
+      if ((rc = set_attrs(&ycol_kernel<T, N, DCT, false>, YC::SMEM, false))) return rc;
+      if ((rc = set_attrs(&zrow_kernel<T, N, DCT, kZrowStep>, ZC::SMEM, false))) return rc;
+      if ((rc = set_attrs(&zrow_kernel<T, N, DCT, kZrowGen>, ZC::SMEM, false))) return rc;
+    }
     return SH_OK;
   }
+
+  // one unclustered kernel of the split plane pass
+  template <class K, class A>
+  int launch_flat(K kern, unsigned grid, unsigned threads, size_t smem, const A& args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = use_pdl ? 1 : 0;
+    SHB_CUDA(cudaLaunchKernelEx(&cfg, kern, args));
+    ++launches;
+    return SH_OK;
+  }
+
+  // The plane pass of a step: psi from its partial a.src, N(psi) and the
+  // diagnostics of a.flags, the partial of N to a.dst.
+  int plane_step(const PlaneArgs<T>& a, int reps = 0) {
+    if constexpr (kSplit) {
+      if (slab) {
+        const int planes = N * (reps > 0 ? reps : p.batch);
+        const bool gen = a.flags != 0 || a.kwall > 0 || p.w_mid != 0.0;
+        int rc;
+        for (int p0 = 0; p0 < planes; p0 += slab_planes) {
+          const int np = std::min(slab_planes, planes - p0);
+          YcolArgs<T> yi{a.src + size_t(p0) * FP, slab, lt};
+          if ((rc = launch_flat(&ycol_kernel<T, N, DCT, true>, np * YC::TILES, YC::THREADS, YC::SMEM, yi))) return rc;
+          ZrowArgs<T> z{};
+          z.slab = slab;
+          z.lt = lt;
+          z.pp = a.pp;
+          z.flags = a.flags;
+          z.plane0 = p0;
+          z.psi_out = a.psi_out;
+          z.psi_old = a.psi_old;
+          z.red = a.red;
+          z.real_out = a.real_out;
+          z.wall = a.wall;
+          z.lperp = a.lperp;
+          z.kwall = a.kwall;
+          if (gen)
+            rc = launch_flat(&zrow_kernel<T, N, DCT, kZrowGen>, np * ZC::BLOCKS, ZC::THREADS, ZC::SMEM, z);
+          else
+            rc = launch_flat(&zrow_kernel<T, N, DCT, kZrowStep>, np * ZC::BLOCKS, ZC::THREADS, ZC::SMEM, z);
+          if (rc) return rc;
+          YcolArgs<T> yf{slab, a.dst + size_t(p0) * FP, lt};
+          if ((rc = launch_flat(&ycol_kernel<T, N, DCT, false>, np * YC::TILES, YC::THREADS, YC::SMEM, yf))) return rc;
+        }
+        return SH_OK;
+      }
+    }
+    return launch_plane<kPlaneStep>(a, reps);
+  }
+  // CTAs per replica that plane_step writes partial sums for
+  int plane_step_blocks() const { return N * (kSplit && slab ? ZC::BLOCKS : CL); }
 
   template <int MODE>
   int launch_plane(const PlaneArgs<T>& a, int reps = 0) {
@@ -517,10 +605,10 @@ struct Solver final : SolverBase {
     return a;
   }
 
-  int finalize(int what, double* out) {
+  int finalize(int what, double* out, int plane_blocks) {
     const double dv = p.dx * p.dx * p.dx;
     const double norm = DCT ? 1.0 / (8.0 * double(N) * N * N) : 1.0 / (double(N) * N * N);
-    finalize_kernel<<<p.batch, 256, 0, stream>>>(d_red_plane, N * CL, d_red_spec, QC::TILES, what, dv, norm,
+    finalize_kernel<<<p.batch, 256, 0, stream>>>(d_red_plane, plane_blocks, d_red_spec, QC::TILES, what, dv, norm,
                                                   p.alpha, p.dt, out);
     SHB_CUDA(cudaGetLastError());
     ++launches;
@@ -634,7 +722,7 @@ struct Solver final : SolverBase {
       a.src = P + off;
       a.dst = Nt + off;
       a.pp.eps = d_eps + r0;
-      if ((rc = launch_plane<kPlaneStep>(a, g))) return rc;
+      if ((rc = plane_step(a, g))) return rc;
     }
     return SH_OK;
   }
@@ -756,7 +844,7 @@ struct Solver final : SolverBase {
           a.flags |= kFlRealOut;
           a.real_out = hist_real + size_t(hist_pos + 1) * size_t(p.batch) * N * N * N;
         }
-        if ((rc = launch_plane<kPlaneStep>(a))) return rc;
+        if ((rc = plane_step(a))) return rc;
       }
       if (prof_ms) {
         float t0, t1;
@@ -767,9 +855,11 @@ struct Solver final : SolverBase {
         prof_ms[0] += t0;
         prof_ms[1] += t1;
       }
-      if (trace && (rc = finalize(0, d_trace + size_t(s) * p.batch))) return rc;
+      // advected steps sum in psi_lpsi_real's plane pass, the others in plane_step
+      const int pb = p.advection ? N * CL : plane_step_blocks();
+      if (trace && (rc = finalize(0, d_trace + size_t(s) * p.batch, pb))) return rc;
       if (l1_now) {
-        if ((rc = finalize(1, d_scalar))) return rc;
+        if ((rc = finalize(1, d_scalar, pb))) return rc;
         ++l1_count;
       }
       ++steps;
@@ -922,7 +1012,7 @@ struct Solver final : SolverBase {
     b.src = P;
     b.flags = kFlEnergy;
     if ((rc = launch_pencil<kPencilEnergy>(b))) return rc;
-    if ((rc = finalize(0, d_scalar))) return rc;
+    if ((rc = finalize(0, d_scalar, N * CL))) return rc;
     SHB_CUDA(cudaMemcpyAsync(host, d_scalar, p.batch * sizeof(double), cudaMemcpyDeviceToHost, stream));
     SHB_CUDA(cudaStreamSynchronize(stream));
     return SH_OK;
