@@ -35,6 +35,7 @@ enum PlaneMode : int {
   kPlaneInvMulFwd = 6,  // inverse of (mult x src) -> real_out; times real_in[0]; forward -> dst
   kPlaneAdvN = 7,       // N(real_in[0]) - sum_c (inverse of src3[c]) real_in[1+c]; forward -> dst
   kPlaneMulFwd = 8,     // real_in[0] real_in[1] (times the signs of sign_axes) forward -> dst
+  kPlaneStepLean = 9,   // kPlaneStep without flags and penalties (flat_kernel.cuh)
 };
 // spectral multiplier applied to the partial spectrum as the plane is loaded
 // kMulSinDy (Neumann): the sine series of d/dy as reversed coefficients,
@@ -149,6 +150,7 @@ struct PlaneArgs {
   double* red;            // per-CTA partial sums [rep][grid.x][3]
   int* timeout;           // set when a bounded wait on a cluster exchange gave up
   const cplx<T>* tw;      // twiddle table [forward | inverse | quarter-wave]
+  const cplx<T>* lt;      // line tables (flat_kernel.cuh)
   PointParams pp;
   int flags;
   // real-field modes: wavenumber table, multiplier, real inputs / output

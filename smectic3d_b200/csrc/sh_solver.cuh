@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/smectic_b200.h"
+#include "flat_kernel.cuh"
 #include "pencil_kernel.cuh"
 #include "plane_kernel.cuh"
 #include "split_kernel.cuh"
@@ -274,8 +275,16 @@ struct Solver final : SolverBase {
     return pp;
   }
 
+  // planes that fit one CTA run in the one-CTA form
+  using LC = FlatCfg<T, N, DCT>;
+  static constexpr bool kFlat = CL == 1 && LC::ok;
+  static constexpr int kPlaneThreads = kFlat ? LC::THREADS : PC::THREADS;
+  static constexpr size_t kPlaneSmem = kFlat ? LC::SMEM : PC::SMEM;
   template <int MODE>
-  static constexpr auto plane_fn() { return &plane_kernel<T, N, CL, DCT, MODE>; }
+  static constexpr auto plane_fn() {
+    if constexpr (kFlat) return &flat_kernel<T, N, DCT, MODE>;
+    else return &plane_kernel<T, N, CL, DCT, MODE>;
+  }
   template <int MODE>
   static constexpr auto pencil_fn() { return &pencil_kernel<T, N, DCT, MODE, TKV>; }
 
@@ -394,10 +403,10 @@ struct Solver final : SolverBase {
     SHB_CUDA(cudaMemcpy(qs, hqs.data(), N * sizeof(T), cudaMemcpyHostToDevice));
     SHB_CUDA(cudaMemcpy(qds, hqds.data(), N * sizeof(double), cudaMemcpyHostToDevice));
     int rc;
-    if ((rc = set_attrs(plane_fn<kPlaneStep>(), PC::SMEM, true))) return rc;
-    if ((rc = set_attrs(plane_fn<kPlaneInit>(), PC::SMEM, true))) return rc;
-    if ((rc = set_attrs(plane_fn<kPlaneGetPsi>(), PC::SMEM, true))) return rc;
-    if ((rc = set_attrs(plane_fn<kPlaneInvReal>(), PC::SMEM, true))) return rc;
+    if ((rc = set_attrs(plane_fn<kPlaneStep>(), kPlaneSmem, true))) return rc;
+    if ((rc = set_attrs(plane_fn<kPlaneInit>(), kPlaneSmem, true))) return rc;
+    if ((rc = set_attrs(plane_fn<kPlaneGetPsi>(), kPlaneSmem, true))) return rc;
+    if ((rc = set_attrs(plane_fn<kPlaneInvReal>(), kPlaneSmem, true))) return rc;
     if ((rc = set_pencil_attrs<kPencilStep>())) return rc;
     if constexpr (sizeof(T) == 4) {
       if ((rc = set_pencil_attrs<kPencilStepU64>())) return rc;
@@ -414,10 +423,13 @@ struct Solver final : SolverBase {
     if ((rc = set_pencil_attrs<kPencilAdjInit>())) return rc;
     if ((rc = set_pencil_attrs<kPencilAdj>())) return rc;
     if ((rc = set_pencil_attrs<kPencilAdjOut>())) return rc;
-    if ((rc = set_attrs(plane_fn<kPlaneAdj>(), PC::SMEM, true))) return rc;
-    if ((rc = set_attrs(plane_fn<kPlaneInvMulFwd>(), PC::SMEM, true))) return rc;
-    if ((rc = set_attrs(plane_fn<kPlaneAdvN>(), PC::SMEM, true))) return rc;
-    if ((rc = set_attrs(plane_fn<kPlaneMulFwd>(), PC::SMEM, true))) return rc;
+    if ((rc = set_attrs(plane_fn<kPlaneAdj>(), kPlaneSmem, true))) return rc;
+    if ((rc = set_attrs(plane_fn<kPlaneInvMulFwd>(), kPlaneSmem, true))) return rc;
+    if ((rc = set_attrs(plane_fn<kPlaneAdvN>(), kPlaneSmem, true))) return rc;
+    if ((rc = set_attrs(plane_fn<kPlaneMulFwd>(), kPlaneSmem, true))) return rc;
+    if constexpr (kFlat) {
+      if ((rc = set_attrs(plane_fn<kPlaneStepLean>(), kPlaneSmem, true))) return rc;
+    }
     if constexpr (kSplit) {
       if ((rc = set_attrs(&ycol_kernel<T, N, DCT, true>, YC::SMEM, false))) return rc;
       if ((rc = set_attrs(&ycol_kernel<T, N, DCT, false>, YC::SMEM, false))) return rc;
@@ -481,6 +493,9 @@ struct Solver final : SolverBase {
         return SH_OK;
       }
     }
+    if constexpr (kFlat) {
+      if (a.flags == 0 && a.kwall == 0 && p.w_mid == 0.0) return launch_plane<kPlaneStepLean>(a, reps);
+    }
     return launch_plane<kPlaneStep>(a, reps);
   }
   // CTAs per replica that plane_step writes partial sums for
@@ -501,8 +516,8 @@ struct Solver final : SolverBase {
     for (int i = 0; i < ncomp; ++i) pl.c[i] = as[i];
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(N * CL, reps > 0 ? reps : p.batch, ncomp);
-    cfg.blockDim = dim3(PC::THREADS, 1, 1);
-    cfg.dynamicSmemBytes = PC::SMEM;
+    cfg.blockDim = dim3(kPlaneThreads, 1, 1);
+    cfg.dynamicSmemBytes = kPlaneSmem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     unsigned na = 0;
@@ -548,14 +563,14 @@ struct Solver final : SolverBase {
     int dev = 0, sms = 0, pb = 0, qb = 0, nc = 0;
     SHB_CUDA(cudaGetDevice(&dev));
     SHB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    SHB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pb, plane_fn<kPlaneStep>(), PC::THREADS, PC::SMEM));
+    SHB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pb, plane_fn<kPlaneStep>(), kPlaneThreads, kPlaneSmem));
     SHB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&qb, pencil_fn<kPencilStep>(), QC::THREADS,
                                                            QC::smem(kPencilStep)));
     if (CL > 1) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(N * CL, p.batch, 1);
-      cfg.blockDim = dim3(PC::THREADS, 1, 1);
-      cfg.dynamicSmemBytes = PC::SMEM;
+      cfg.blockDim = dim3(kPlaneThreads, 1, 1);
+      cfg.dynamicSmemBytes = kPlaneSmem;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = CL;
@@ -585,6 +600,7 @@ struct Solver final : SolverBase {
     // clustered plane passes run in several waves: prefetch a later wave's planes
     a.pf_dist = CL > 1 ? SHB_PLANE_PF : 0;
     a.tw = tw;
+    a.lt = lt;
     a.pp = point_params();
     a.red = d_red_plane;
     a.timeout = d_flag + 1;
