@@ -670,19 +670,35 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
       }
     }
   } else if constexpr (MODE == kPencilStokes) {
-    // The three stress components go forward one after the other; the first two
-    // spectra wait in shared memory, the projector runs in registers, and the
-    // three velocity components go back.
+    // The three stress components go forward one after the other, the second and the
+    // third on their way into shared memory meanwhile; there the finished spectra
+    // take the place of the lines (every thread reads and writes its own slots only).
+    // The projector runs in registers, and the three velocity components go back.
     cplx<T>* keep[2] = {aside, aside + size_t(TK) * N};
     constexpr int TH = Cfg::THREADS;
-#pragma unroll 1
-    for (int comp = 0; comp < 3; ++comp) {
-      Ops::load(v, a.s3[comp] + line, t);
-      Ops::forward(v, x, t, tw, comp > 0);
-      if (comp < 2) {
 #pragma unroll
-        for (int s = 0; s < E; ++s) keep[comp][s * TH] = v[s];
+    for (int m = 0; m < 2; ++m) {
+      const cplx<T>* src = a.s3[m + 1] + line;
+#pragma unroll
+      for (int s = 0; s < E; ++s)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(keep[m] + s * TH)),
+                     "l"(src + size_t(real_pos<N, DCT>(LineIdx<N>::a_elem(t, s))) * FP), "n"(int(sizeof(cplx<T>)))
+                     : "memory");
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    Ops::load(v, a.s3[0] + line, t);
+    Ops::forward(v, x, t, tw, false);
+#pragma unroll 1
+    for (int m = 0; m < 2; ++m) {
+      if (m == 0) asm volatile("cp.async.wait_group 1;" ::: "memory");
+      else asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+      for (int s = 0; s < E; ++s) {
+        const cplx<T> u = keep[m][s * TH];
+        keep[m][s * TH] = v[s];
+        v[s] = u;
       }
+      Ops::forward(v, x, t, tw, true);
     }
     const T ce = T(1.0 / a.pp.eta_rho);
     if constexpr (DCT) {

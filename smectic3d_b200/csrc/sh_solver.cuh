@@ -197,6 +197,7 @@ struct Solver final : SolverBase {
   cplx<T>* Psc = nullptr;
   bool real_fields_current = false;
   bool u_real_current = false;
+  bool lpsi_current = false;
   // adjoint work buffers, kept for the handle's lifetime once allocated
   struct AdjBufs {
     cplx<T>* ck = nullptr;   // checkpoints: nseg states x {W, P, Nt}
@@ -253,8 +254,7 @@ struct Solver final : SolverBase {
   size_t field_elems() const { return size_t(p.batch) * N * FP; }
 
   // planes too large for one CTA go through the split passes
-    static constexpr bool kSplit = N >= 256;
-  static constexpr size_t kSlabBytes = size_t(64) << 20;
+  static constexpr bool kSplit = N >= 256;
   using YC = YcolCfg<T, N, DCT>;
   using ZC = ZrowCfg<T, N, DCT>;
 
@@ -323,16 +323,6 @@ struct Solver final : SolverBase {
     SHB_CUDA(dev_malloc(&W, fe * sizeof(cplx<T>)));
     SHB_CUDA(dev_malloc(&P, fe * sizeof(cplx<T>)));
     SHB_CUDA(dev_malloc(&Nt, fe * sizeof(cplx<T>)));
-    if constexpr (kSplit) {
-      constexpr size_t plane_bytes = size_t(YC::SP) * sizeof(cplx<T>);
-      const long long planes = (long long)p.batch * N;
-      slab_planes = int(std::min<long long>(planes, std::max<long long>(1, kSlabBytes / plane_bytes)));
-      if (dev_malloc(&slab, slab_planes * plane_bytes) != cudaSuccess) {
-        // the fields themselves fit: keep the clustered plane pass, which needs no slab
-        cudaGetLastError();
-        slab = nullptr;
-      }
-    }
     if (p.advection) {
       // periodic: partials of psi, i q_x psi and opSH psi; Neumann: of psi and
       // opSH psi (its gradient is a difference stencil in real space)
@@ -433,17 +423,58 @@ struct Solver final : SolverBase {
     if constexpr (kSplit) {
       if ((rc = set_attrs(&ycol_kernel<T, N, DCT, true>, YC::SMEM, false))) return rc;
       if ((rc = set_attrs(&ycol_kernel<T, N, DCT, false>, YC::SMEM, false))) return rc;
-      if ((rc = set_attrs(&zrow_kernel<T, N, DCT, kZrowStep>, ZC::SMEM, false))) return rc;
-      if ((rc = set_attrs(&zrow_kernel<T, N, DCT, kZrowGen>, ZC::SMEM, false))) return rc;
+      if ((rc = set_zrow_attrs<kZrowStep>())) return rc;
+      if ((rc = set_zrow_attrs<kZrowGen>())) return rc;
+      if ((rc = set_zrow_attrs<kZrowAdvN>())) return rc;
+      if constexpr (DCT) {
+        if ((rc = set_zrow_attrs<kZrowReal>())) return rc;
+        if ((rc = set_zrow_attrs<kZrowMul>())) return rc;
+      } else {
+        if ((rc = set_attrs(&ycol_kernel<T, N, DCT, true, true>, YC::SMEM, false))) return rc;
+        if ((rc = set_zrow_attrs<kZrowStress>())) return rc;
+      }
+      if ((rc = setup_slab())) return rc;
     }
     return SH_OK;
   }
 
-  // one unclustered kernel of the split plane pass
+  // The slab of the split passes: whole waves of CTAs, so that no pass ends with a
+  // nearly empty one, and small enough to stay in L2.  Plain steps: four waves of the
+  // column pass (74 MB; 512^3 FP64 37 planes).  Advected steps: one wave of the
+  // longest row pass, over kSplitComps fields (256^3 FP32 55 planes, 55 MB).
+  int setup_slab() {
+    int dev = 0, sms = 0, occ = 0;
+    SHB_CUDA(cudaGetDevice(&dev));
+    SHB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    long long planes;
+    if (p.advection) {
+      constexpr int mode = DCT ? int(kZrowAdvN) : int(kZrowStress);
+      SHB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, &zrow_kernel<T, N, DCT, mode>, ZC::THREADS,
+                                                             ZC::smem(mode)));
+      planes = (long long)occ * sms / ZC::BLOCKS;
+    } else {
+      SHB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, &ycol_kernel<T, N, DCT, true>, YC::THREADS, YC::SMEM));
+      planes = 4ll * occ * sms / YC::TILES;
+    }
+    planes = std::max(1ll, std::min(planes, (long long)p.batch * N));
+    const size_t bytes = size_t(planes) * YC::SP * sizeof(cplx<T>) * (p.advection ? kSplitComps : 1);
+    if (dev_malloc(&slab, bytes) != cudaSuccess) {
+      // the fields themselves fit: keep the clustered plane pass, which needs no slab
+      cudaGetLastError();
+      slab = nullptr;
+      return SH_OK;
+    }
+    slab_planes = int(planes);
+    return SH_OK;
+  }
+  template <int MODE>
+  int set_zrow_attrs() { return set_attrs(&zrow_kernel<T, N, DCT, MODE>, ZC::smem(MODE), false); }
+
+  // one kernel of the split plane pass over ``fields`` fields
   template <class K, class A>
-  int launch_flat(K kern, unsigned grid, unsigned threads, size_t smem, const A& args) {
+  int launch_split(K kern, unsigned grid, unsigned fields, unsigned threads, size_t smem, const A& args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.gridDim = dim3(grid, fields, 1);
     cfg.blockDim = dim3(threads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -457,6 +488,48 @@ struct Solver final : SolverBase {
     return SH_OK;
   }
 
+  // y passes of ``nf`` fields over np planes: partials -> slabs, slabs -> partials
+  // (pointers to the first plane); field ``iqy`` is multiplied by i q_y
+  int slab_in(const cplx<T>* const* src, int nf, size_t p0, int np, int iqy = -1) {
+    YcolArgs<T> y{};
+    for (int f = 0; f < nf; ++f) {
+      y.src[f] = src[f] + p0 * FP;
+      y.dst[f] = slab_of(f);
+    }
+    y.lt = lt;
+    y.q = q;
+    y.iqy = iqy;
+    if constexpr (!DCT) {
+      if (iqy >= 0)
+        return launch_split(&ycol_kernel<T, N, DCT, true, true>, np * YC::TILES, nf, YC::THREADS, YC::SMEM, y);
+    }
+    return launch_split(&ycol_kernel<T, N, DCT, true>, np * YC::TILES, nf, YC::THREADS, YC::SMEM, y);
+  }
+  int slab_out(const int* slabs, cplx<T>* const* dst, int nf, size_t p0, int np) {
+    YcolArgs<T> y{};
+    for (int f = 0; f < nf; ++f) {
+      y.src[f] = slab_of(slabs[f]);
+      y.dst[f] = dst[f] + p0 * FP;
+    }
+    y.lt = lt;
+    return launch_split(&ycol_kernel<T, N, DCT, false>, np * YC::TILES, nf, YC::THREADS, YC::SMEM, y);
+  }
+  template <int MODE>
+  int slab_rows(const ZrowArgs<T>& z, int np, int nf = 1) {
+    return launch_split(&zrow_kernel<T, N, DCT, MODE>, np * ZC::BLOCKS, nf, ZC::THREADS, ZC::smem(MODE), z);
+  }
+  cplx<T>* slab_of(int f) const { return slab + size_t(f) * slab_planes * YC::SP; }
+  ZrowArgs<T> zrow_args(int p0) const {
+    ZrowArgs<T> z{};
+    for (int f = 0; f < (p.advection ? kSplitComps : 1); ++f) z.slab[f] = slab_of(f);
+    z.lt = lt;
+    z.pp = point_params();
+    z.q = q;
+    z.plane0 = p0;
+    z.red = d_red_plane;
+    return z;
+  }
+
   // The plane pass of a step: psi from its partial a.src, N(psi) and the
   // diagnostics of a.flags, the partial of N to a.dst.
   int plane_step(const PlaneArgs<T>& a, int reps = 0) {
@@ -464,31 +537,22 @@ struct Solver final : SolverBase {
       if (slab) {
         const int planes = N * (reps > 0 ? reps : p.batch);
         const bool gen = a.flags != 0 || a.kwall > 0 || p.w_mid != 0.0;
+        const int first = 0;
         int rc;
         for (int p0 = 0; p0 < planes; p0 += slab_planes) {
           const int np = std::min(slab_planes, planes - p0);
-          YcolArgs<T> yi{a.src + size_t(p0) * FP, slab, lt};
-          if ((rc = launch_flat(&ycol_kernel<T, N, DCT, true>, np * YC::TILES, YC::THREADS, YC::SMEM, yi))) return rc;
-          ZrowArgs<T> z{};
-          z.slab = slab;
-          z.lt = lt;
+          if ((rc = slab_in(&a.src, 1, p0, np))) return rc;
+          ZrowArgs<T> z = zrow_args(p0);
           z.pp = a.pp;
           z.flags = a.flags;
-          z.plane0 = p0;
           z.psi_out = a.psi_out;
           z.psi_old = a.psi_old;
-          z.red = a.red;
           z.real_out = a.real_out;
           z.wall = a.wall;
           z.lperp = a.lperp;
           z.kwall = a.kwall;
-          if (gen)
-            rc = launch_flat(&zrow_kernel<T, N, DCT, kZrowGen>, np * ZC::BLOCKS, ZC::THREADS, ZC::SMEM, z);
-          else
-            rc = launch_flat(&zrow_kernel<T, N, DCT, kZrowStep>, np * ZC::BLOCKS, ZC::THREADS, ZC::SMEM, z);
-          if (rc) return rc;
-          YcolArgs<T> yf{slab, a.dst + size_t(p0) * FP, lt};
-          if ((rc = launch_flat(&ycol_kernel<T, N, DCT, false>, np * YC::TILES, YC::THREADS, YC::SMEM, yf))) return rc;
+          if ((rc = gen ? slab_rows<kZrowGen>(z, np) : slab_rows<kZrowStep>(z, np))) return rc;
+          if ((rc = slab_out(&first, &a.dst, 1, p0, np))) return rc;
         }
         return SH_OK;
       }
@@ -871,8 +935,7 @@ struct Solver final : SolverBase {
         prof_ms[0] += t0;
         prof_ms[1] += t1;
       }
-      // advected steps sum in psi_lpsi_real's plane pass, the others in plane_step
-      const int pb = p.advection ? N * CL : plane_step_blocks();
+      const int pb = plane_step_blocks();
       if (trace && (rc = finalize(0, d_trace + size_t(s) * p.batch, pb))) return rc;
       if (l1_now) {
         if ((rc = finalize(1, d_scalar, pb))) return rc;
@@ -889,6 +952,9 @@ struct Solver final : SolverBase {
   // stress S = (L psi) grad psi, Stokes velocity u, then
   // N = beta psi^3 - gamma psi^5 (+ penalty) - u.grad psi, forward y,z -> Nt.
   int adv_nonlinear(int diag) {
+    if constexpr (kSplit) {
+      if (slab) return adv_nonlinear_split(diag);
+    }
     if constexpr (DCT) {
       // Neumann box (cosFFT/comet/morphSurfK.cpp:686-898): psi and L psi to real
       // space, grad psi by the wall stencil, S_c = (L psi) d_c psi through the
@@ -957,6 +1023,77 @@ struct Solver final : SolverBase {
       return SH_OK;
     }
   }
+  // the same through the split passes, slab by slab
+  int adv_nonlinear_split(int diag) {
+    int rc;
+    const int planes = N * p.batch;
+    for (int p0 = 0; p0 < planes; p0 += slab_planes) {
+      const int np = std::min(slab_planes, planes - p0);
+      ZrowArgs<T> z = zrow_args(p0);
+      z.flags = diag;
+      z.psi_old = d_stash;
+      z.psi_out = d_stash;
+      if constexpr (DCT) {
+        const cplx<T>* src[2] = {P, PSH};
+        if ((rc = slab_in(src, 2, p0, np))) return rc;
+        z.real_to[0] = R[0];
+        z.real_to[1] = R[4];
+        if ((rc = slab_rows<kZrowReal>(z, np, 2))) return rc;
+      } else {
+        const cplx<T>* src[4] = {P, Px, P, PSH};
+        if ((rc = slab_in(src, 4, p0, np, 2))) return rc;
+        for (int c = 0; c < 3; ++c) z.real_to[c] = R[1 + c];
+        z.real_to[3] = R[0];
+        if ((rc = slab_rows<kZrowStress>(z, np))) return rc;
+        const int back[3] = {1, 2, 0};
+        if ((rc = slab_out(back, S3, 3, p0, np))) return rc;
+      }
+    }
+    const int all[3] = {0, 1, 2};
+    if constexpr (DCT) {
+      grad_wall_kernel<T><<<dim3(4 * 148, p.batch), 256, 0, stream>>>(R[0], R[1], R[2], R[3], N, T(0.5 / p.dx));
+      SHB_CUDA(cudaGetLastError());
+      ++launches;
+      for (int p0 = 0; p0 < planes; p0 += slab_planes) {
+        const int np = std::min(slab_planes, planes - p0);
+        ZrowArgs<T> z = zrow_args(p0);
+        for (int c = 0; c < 3; ++c) z.real_in[c] = R[1 + c];
+        z.real_in[3] = R[4];
+        z.sign_axes = 7;
+        if ((rc = slab_rows<kZrowMul>(z, np, 3))) return rc;
+        if ((rc = slab_out(all, S3, 3, p0, np))) return rc;
+      }
+    }
+    PencilArgs<T> b = pencil_args();
+    for (int c = 0; c < 3; ++c) {
+      b.s3[c] = S3[c];
+      b.u3[c] = S3[c];
+    }
+    if ((rc = launch_pencil<kPencilStokes>(b))) return rc;
+    for (int p0 = 0; p0 < planes; p0 += slab_planes) {
+      const int np = std::min(slab_planes, planes - p0);
+      const cplx<T>* src[3] = {S3[0], S3[1], S3[2]};
+      if ((rc = slab_in(src, 3, p0, np))) return rc;
+      ZrowArgs<T> z = zrow_args(p0);
+      for (int c = 0; c < 3; ++c) z.real_in[c] = R[1 + c];
+      z.real_in[3] = R[0];
+      z.sign_axes = DCT ? 7 : 0;
+      if ((rc = slab_rows<kZrowAdvN>(z, np))) return rc;
+      if ((rc = slab_out(all, &Nt, 1, p0, np))) return rc;
+    }
+    real_fields_current = true;
+    lpsi_current = DCT;  // the periodic stress pass keeps L psi to itself
+    u_real_current = false;
+    return SH_OK;
+  }
+  // L psi of the current state in real space (R[4])
+  int lpsi_real() {
+    PlaneArgs<T> a = plane_args();
+    a.src = PSH;
+    a.real_out = R[4];
+    lpsi_current = true;
+    return launch_plane<kPlaneInvReal>(a);
+  }
   // psi and L psi of the state held in P, PSH to real space (R[0], R[4]), one
   // grid; the diagnostics ``diag`` (L1 monitor, psi stash) ride on psi
   int psi_lpsi_real(int diag) {
@@ -968,6 +1105,7 @@ struct Solver final : SolverBase {
     st[0].psi_out = d_stash;
     st[1].src = PSH;
     st[1].real_out = R[4];
+    lpsi_current = true;
     return launch_plane_sets<kPlaneInvReal>(st, 2);
   }
   // velocity of the current state in real space (R[5..7]) from its partials in S3
@@ -1465,6 +1603,7 @@ struct Solver final : SolverBase {
         for (auto& d : d_surf) SHB_CUDA(dev_malloc(&d, nc * sizeof(double)));
       }
       if (!real_fields_current && (rc = adv_nonlinear(0))) return rc;
+      if (!lpsi_current && (rc = lpsi_real())) return rc;
       if (!u_real_current && (rc = velocity_real())) return rc;
       // second derivatives of psi^n: psi_xx = C2R(-q_x^2 psihat), psi_yy, psi_xy
       PencilArgs<T> b = pencil_args();
