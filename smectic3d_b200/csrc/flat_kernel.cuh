@@ -37,7 +37,9 @@ struct FlatCfg {
 
 template <typename T, int N, bool DCT, int MODE>
 __global__ void __launch_bounds__(FlatCfg<T, N, DCT>::THREADS,
-                                  MODE == kPlaneStepLean || MODE == kPlaneAdj ? FlatCfg<T, N, DCT>::MIN_BLOCKS : 1)
+                                  MODE == kPlaneStepLean || MODE == kPlaneStepHist || MODE == kPlaneAdj
+                                      ? FlatCfg<T, N, DCT>::MIN_BLOCKS
+                                      : 1)
 flat_kernel(const __grid_constant__ PlaneLaunch<T> pl) {
   const PlaneArgs<T>& a = pl.c[plane_multi(MODE) ? blockIdx.z : 0];
   using Cfg = FlatCfg<T, N, DCT>;
@@ -138,9 +140,10 @@ flat_kernel(const __grid_constant__ PlaneLaunch<T> pl) {
     }
   };
 
-  if constexpr (MODE == kPlaneStepLean) {
+  if constexpr (MODE == kPlaneStepLean || MODE == kPlaneStepHist) {
     columns_in(a.src + plane_off, kMulNone, nullptr, kMulNone, false);
     rows_in();
+    if constexpr (MODE == kPlaneStepHist) S::real_store(v, rt, a.real_out, ra, rb);
     S::nonlin(v, a.pp);
     rows_out(a.dst + plane_off, true);
   } else if constexpr (MODE == kPlaneStep || MODE == kPlaneGetPsi || MODE == kPlaneInvReal || MODE == kPlaneAdj ||

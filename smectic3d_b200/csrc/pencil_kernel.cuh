@@ -38,6 +38,8 @@ enum PencilMode : int {
   kPencilStepU64 = 11, // the step of FP32 fields with the CNAB2 multipliers and update in FP64
   kPencilStepGen = 12, // the step with what kPencilStep leaves out: IMEX Euler, the energy, psihat out
   kPencilStepU64Gen = 13,  // the same for kPencilStepU64
+  kPencilStepAdvGen = 14,  // the same for kPencilStepAdv
+  kPencilStepSpec = 15,    // kPencilStep that keeps psihat^{n+1} in spec_out (the adjoint's recompute)
 };
 // multiplier of kPencilXMul
 enum XMulKind : int {
@@ -50,7 +52,7 @@ enum XMulKind : int {
 // tiles of shared memory a pencil mode uses (the exchange, a spectrum kept
 // aside, Stokes components)
 __host__ __device__ constexpr int pencil_sets(int mode) {
-  return mode == kPencilStokes ? 3 : ((mode == kPencilStepAdv || mode == kPencilInitAdv || mode == kPencilInit) ? 2 : 1);
+  return mode == kPencilStokes ? 3 : ((mode == kPencilStepAdv || mode == kPencilStepAdvGen || mode == kPencilInitAdv || mode == kPencilInit) ? 2 : 1);
 }
 
 // TKV: lines per CTA (the tile), 0 = the default of 16 (FP32) or 8 (FP64)
@@ -291,7 +293,7 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
   const bool want_energy = (a.flags & kFlEnergy) != 0;
   grid_dependency_wait();
 
-  if constexpr (MODE == kPencilStep || MODE == kPencilStepU64) {
+  if constexpr (MODE == kPencilStep || MODE == kPencilStepU64 || MODE == kPencilStepAdv || MODE == kPencilStepSpec) {
     // CNAB2 and nothing else: this kernel is bound by the instructions it issues
     // and fetches, so what only some runs ask for (kPencilStepGen) stays out of it
     cplx<T>* w = a.w + line;
@@ -369,12 +371,13 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
           wv = cfma<T>(c1, pn, cmul2<T>(both<T>(-h), nh));
         }
         finite = cfma<T>(pn, both<T>(T(0)), finite);
+        if constexpr (MODE == kPencilStepSpec) a.spec_out[line + size_t(Ops::kx_of(t, s)) * FP] = pn;
         w[size_t(Ops::kx_of(t, s)) * FP] = wv;
         v[s] = cscale<T>(pn, scale);
       }
     }
     if (!(finite.x == T(0) && finite.y == T(0))) *a.nonfinite = 1;
-  } else if constexpr (MODE == kPencilStepGen || MODE == kPencilStepU64Gen || MODE == kPencilStepAdv) {
+  } else if constexpr (MODE == kPencilStepGen || MODE == kPencilStepU64Gen || MODE == kPencilStepAdvGen) {
     cplx<T>* w = a.w + line;
     Ops::load(v, a.src + line, t);
     Ops::forward(v, x, t, tw, false);
@@ -716,7 +719,7 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
         const cplx<T> px = keep[0][s * TH], py = keep[1][s * TH], pz = v[s];
         // .x holds kz, .y holds kz + 1
         const T m0 = sx * sx + sy * sy + sz0 * sz0, m1 = sx * sx + sy * sy + sz1 * sz1;
-        const T i0 = T(1) / m0, i1 = T(1) / m1;
+        const T i0 = rcp2(m0), i1 = rcp2(m1);
         const T c0 = scale * ce * i0, c1 = scale * ce * i1;
         const T d0 = sx * px.x + sy * py.x + sz0 * pz.x;
         const T d1 = sx * px.y + sy * py.y + sz1 * pz.y;
@@ -733,7 +736,7 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
         const cplx<T> sx = keep[0][s * TH], sy = keep[1][s * TH], sz = v[s];
         cplx<T> ux = mk<T>(T(0), T(0)), uy = ux, uz = ux;
         if (mq2 != T(0)) {
-          const T inv = T(1) / mq2;
+          const T inv = rcp2(mq2);
           const T cm1 = scale * ce * inv;
           const cplx<T> dot = mk<T>(qx * sx.x + qy * sy.x + qz0 * sz.x, qx * sx.y + qy * sy.y + qz0 * sz.y);
           ux = mk<T>(cm1 * (sx.x - qx * inv * dot.x), cm1 * (sx.y - qx * inv * dot.y));
@@ -780,11 +783,12 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
     }
   }
 
-  if constexpr (MODE == kPencilStep || MODE == kPencilStepGen || MODE == kPencilStepU64 || MODE == kPencilStepU64Gen || MODE == kPencilInit || MODE == kPencilXMul ||
+  if constexpr (MODE == kPencilStep || MODE == kPencilStepSpec || MODE == kPencilStepGen || MODE == kPencilStepU64 ||
+                MODE == kPencilStepU64Gen || MODE == kPencilInit || MODE == kPencilXMul ||
                 MODE == kPencilAdjInit || MODE == kPencilAdj || MODE == kPencilAdjOut) {
     Ops::inverse(v, x, t, tw, MODE != kPencilAdjOut);
     Ops::store(v, a.dst + line, t);
-  } else if constexpr (MODE == kPencilStepAdv || MODE == kPencilInitAdv) {
+  } else if constexpr (MODE == kPencilStepAdv || MODE == kPencilStepAdvGen || MODE == kPencilInitAdv) {
     // v = scale psihat^{n+1}; emit its partial, one inverse x transform each, and
     //   periodic: those of i q_x v and opSH v (periodicFFT/pf3d.cpp:404-407)
     //   Neumann, where asked: those of -q_x^2 v (the x half of the substrate's
@@ -817,7 +821,7 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
     }
   }
 
-  if (want_energy && (MODE == kPencilStepGen || MODE == kPencilStepU64Gen || MODE == kPencilStepAdv ||
+  if (want_energy && (MODE == kPencilStepGen || MODE == kPencilStepU64Gen || MODE == kPencilStepAdvGen ||
                       MODE == kPencilEnergy)) {
     const double tot = block_sum(acc.s, scratch);
     if (threadIdx.x == 0) a.red[size_t(rep) * gridDim.x + blockIdx.x] = tot;

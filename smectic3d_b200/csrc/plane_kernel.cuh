@@ -36,6 +36,7 @@ enum PlaneMode : int {
   kPlaneAdvN = 7,       // N(real_in[0]) - sum_c (inverse of src3[c]) real_in[1+c]; forward -> dst
   kPlaneMulFwd = 8,     // real_in[0] real_in[1] (times the signs of sign_axes) forward -> dst
   kPlaneStepLean = 9,   // kPlaneStep without flags and penalties (flat_kernel.cuh)
+  kPlaneStepHist = 10,  // kPlaneStepLean that writes psi to real_out (flat_kernel.cuh)
 };
 // spectral multiplier applied to the partial spectrum as the plane is loaded
 // kMulSinDy (Neumann): the sine series of d/dy as reversed coefficients,

@@ -303,8 +303,14 @@ struct Solver final : SolverBase {
       if (p.precision == SH_FP32_UPDATE64)
         return gen ? launch_pencil<kPencilStepU64Gen>(b, reps) : launch_pencil<kPencilStepU64>(b, reps);
     }
+    if (p.scheme == kCNAB2 && b.flags == kFlSpecOut) return launch_pencil<kPencilStepSpec>(b, reps);
     if (gen) return launch_pencil<kPencilStepGen>(b, reps);
     return launch_pencil<kPencilStep>(b, reps);
+  }
+
+  int launch_pencil_step_adv(const PencilArgs<T>& b) {
+    if (p.scheme != kCNAB2 || b.flags != 0) return launch_pencil<kPencilStepAdvGen>(b);
+    return launch_pencil<kPencilStepAdv>(b);
   }
 
   // a pencil mode whose shared memory does not fit a CTA is never launched
@@ -403,9 +409,11 @@ struct Solver final : SolverBase {
       if ((rc = set_pencil_attrs<kPencilStepU64Gen>())) return rc;
     }
     if ((rc = set_pencil_attrs<kPencilStepGen>())) return rc;
+    if ((rc = set_pencil_attrs<kPencilStepSpec>())) return rc;
     if ((rc = set_pencil_attrs<kPencilInit>())) return rc;
     if ((rc = set_pencil_attrs<kPencilEnergy>())) return rc;
     if ((rc = set_pencil_attrs<kPencilStepAdv>())) return rc;
+    if ((rc = set_pencil_attrs<kPencilStepAdvGen>())) return rc;
     if ((rc = set_pencil_attrs<kPencilInitAdv>())) return rc;
     if ((rc = set_pencil_attrs<kPencilStokes>())) return rc;
     if ((rc = set_pencil_attrs<kPencilXMul>())) return rc;
@@ -419,6 +427,7 @@ struct Solver final : SolverBase {
     if ((rc = set_attrs(plane_fn<kPlaneMulFwd>(), kPlaneSmem, true))) return rc;
     if constexpr (kFlat) {
       if ((rc = set_attrs(plane_fn<kPlaneStepLean>(), kPlaneSmem, true))) return rc;
+      if ((rc = set_attrs(plane_fn<kPlaneStepHist>(), kPlaneSmem, true))) return rc;
     }
     if constexpr (kSplit) {
       if ((rc = set_attrs(&ycol_kernel<T, N, DCT, true>, YC::SMEM, false))) return rc;
@@ -426,8 +435,9 @@ struct Solver final : SolverBase {
       if ((rc = set_zrow_attrs<kZrowStep>())) return rc;
       if ((rc = set_zrow_attrs<kZrowGen>())) return rc;
       if ((rc = set_zrow_attrs<kZrowAdvN>())) return rc;
+      if ((rc = set_zrow_attrs<kZrowReal>())) return rc;
+      if ((rc = set_zrow_attrs<kZrowInit>())) return rc;
       if constexpr (DCT) {
-        if ((rc = set_zrow_attrs<kZrowReal>())) return rc;
         if ((rc = set_zrow_attrs<kZrowMul>())) return rc;
       } else {
         if ((rc = set_attrs(&ycol_kernel<T, N, DCT, true, true>, YC::SMEM, false))) return rc;
@@ -505,10 +515,10 @@ struct Solver final : SolverBase {
     }
     return launch_split(&ycol_kernel<T, N, DCT, true>, np * YC::TILES, nf, YC::THREADS, YC::SMEM, y);
   }
-  int slab_out(const int* slabs, cplx<T>* const* dst, int nf, size_t p0, int np) {
+  int slab_out(const int* slabs, cplx<T>* const* dst, int nf, size_t p0, int np, int field_planes = 0) {
     YcolArgs<T> y{};
     for (int f = 0; f < nf; ++f) {
-      y.src[f] = slab_of(slabs[f]);
+      y.src[f] = slab + size_t(slabs[f]) * (field_planes ? field_planes : slab_planes) * YC::SP;
       y.dst[f] = dst[f] + p0 * FP;
     }
     y.lt = lt;
@@ -521,7 +531,7 @@ struct Solver final : SolverBase {
   cplx<T>* slab_of(int f) const { return slab + size_t(f) * slab_planes * YC::SP; }
   ZrowArgs<T> zrow_args(int p0) const {
     ZrowArgs<T> z{};
-    for (int f = 0; f < (p.advection ? kSplitComps : 1); ++f) z.slab[f] = slab_of(f);
+    for (int f = 0; f < kSplitComps; ++f) z.slab[f] = slab_of(f);
     z.lt = lt;
     z.pp = point_params();
     z.q = q;
@@ -558,10 +568,38 @@ struct Solver final : SolverBase {
       }
     }
     if constexpr (kFlat) {
-      if (a.flags == 0 && a.kwall == 0 && p.w_mid == 0.0) return launch_plane<kPlaneStepLean>(a, reps);
+      if (a.kwall == 0 && p.w_mid == 0.0) {
+        if (a.flags == 0) return launch_plane<kPlaneStepLean>(a, reps);
+        if (a.flags == kFlRealOut) return launch_plane<kPlaneStepHist>(a, reps);
+      }
     }
     return launch_plane<kPlaneStep>(a, reps);
   }
+  // real psi a.psi_in -> partials of psi (a.dst2) and of N(psi) (a.dst)
+  int plane_init(const PlaneArgs<T>& a) {
+    if constexpr (kSplit) {
+      if (slab) {
+        const int planes = N * p.batch, all[2] = {0, 1};
+        cplx<T>* const dst[2] = {a.dst2, a.dst};
+        int rc;
+        for (int p0 = 0, step = two_field_planes(); p0 < planes; p0 += step) {
+          const int np = std::min(step, planes - p0);
+          ZrowArgs<T> z = zrow_args(p0);
+          z.psi_in = a.psi_in;
+          z.wall = a.wall;
+          z.lperp = a.lperp;
+          z.kwall = a.kwall;
+          if (!p.advection) z.slab[1] = slab + size_t(step) * YC::SP;
+          if ((rc = slab_rows<kZrowInit>(z, np, 2))) return rc;
+          if ((rc = slab_out(all, dst, 2, p0, np, p.advection ? slab_planes : step))) return rc;
+        }
+        return SH_OK;
+      }
+    }
+    return launch_plane<kPlaneInit>(a);
+  }
+  // planes of two fields that the slab of a plain handle (one field) holds
+  int two_field_planes() const { return p.advection ? slab_planes : std::max(1, slab_planes / 2); }
   // CTAs per replica that plane_step writes partial sums for
   int plane_step_blocks() const { return N * (kSplit && slab ? ZC::BLOCKS : CL); }
 
@@ -730,7 +768,7 @@ struct Solver final : SolverBase {
       // N(psi^0) carries the substrate term of psi^0 (cosFFT/comet/cosNoAdvMorph.cpp:486-529):
       // a first pass yields psi^0's partials, hence its in-plane Laplacian; the second
       // pass builds N-hat^{-1} and W^0 with it
-      if ((rc = launch_plane<kPlaneInit>(a))) return rc;
+      if ((rc = plane_init(a))) return rc;
       b.dst_x = Pxx;
       if ((rc = launch_pencil<kPencilInitAdv>(b))) return rc;
       if ((rc = substrate_lperp())) return rc;
@@ -738,10 +776,10 @@ struct Solver final : SolverBase {
       a.psi_in = d_psi;
       a.dst2 = P;
       a.dst = Nt;
-      if ((rc = launch_plane<kPlaneInit>(a))) return rc;
+      if ((rc = plane_init(a))) return rc;
       if ((rc = launch_pencil<kPencilInitAdv>(b))) return rc;
     } else {
-      if ((rc = launch_plane<kPlaneInit>(a))) return rc;
+      if ((rc = plane_init(a))) return rc;
       if (p.advection) {
         b.dst_x = DCT ? nullptr : Px;
         b.dst_sh = PSH;
@@ -901,13 +939,13 @@ struct Solver final : SolverBase {
       if (p.advection) {
         b.dst_x = DCT ? nullptr : Px;
         b.dst_sh = PSH;
-        if ((rc = launch_pencil<kPencilStepAdv>(b))) return rc;
+        if ((rc = launch_pencil_step_adv(b))) return rc;
         if (prof_ms) SHB_CUDA(cudaEventRecord(prof_ev[1], stream));
         if ((rc = adv_nonlinear(diag))) return rc;
       } else {
         if (kwall > 0) {  // Neumann substrate: also the -q_x^2 partial, then the in-plane Laplacian
           b.dst_x = Pxx;
-          if ((rc = launch_pencil<kPencilStepAdv>(b))) return rc;
+          if ((rc = launch_pencil_step_adv(b))) return rc;
           if (prof_ms) SHB_CUDA(cudaEventRecord(prof_ev[1], stream));
           if ((rc = substrate_lperp())) return rc;
         } else {
@@ -1152,6 +1190,21 @@ struct Solver final : SolverBase {
   }
 
   int plane_getpsi(bool write_psi, bool energy) {
+    if constexpr (kSplit) {
+      if (slab) {
+        int rc;
+        for (int p0 = 0; p0 < N * p.batch; p0 += slab_planes) {
+          const int np = std::min(slab_planes, N * p.batch - p0);
+          const cplx<T>* src = P;
+          if ((rc = slab_in(&src, 1, p0, np))) return rc;
+          ZrowArgs<T> z = zrow_args(p0);
+          z.flags = (write_psi ? kFlPsiOut : 0) | (energy ? kFlEnergy : 0);
+          z.psi_out = d_psi;
+          if ((rc = slab_rows<kZrowReal>(z, np))) return rc;
+        }
+        return SH_OK;
+      }
+    }
     PlaneArgs<T> a = plane_args();
     a.src = P;
     a.psi_out = d_psi;
@@ -1166,7 +1219,7 @@ struct Solver final : SolverBase {
     b.src = P;
     b.flags = kFlEnergy;
     if ((rc = launch_pencil<kPencilEnergy>(b))) return rc;
-    if ((rc = finalize(0, d_scalar, N * CL))) return rc;
+    if ((rc = finalize(0, d_scalar, plane_step_blocks()))) return rc;
     SHB_CUDA(cudaMemcpyAsync(host, d_scalar, p.batch * sizeof(double), cudaMemcpyDeviceToHost, stream));
     SHB_CUDA(cudaStreamSynchronize(stream));
     return SH_OK;
@@ -1407,7 +1460,7 @@ struct Solver final : SolverBase {
         a.psi_in = d_psi;
         a.dst2 = bf.gp;   // partial of lambda^T
         a.dst = bf.mp;    // (the N of lambda^T, unused scratch)
-        ADJ_RC(launch_plane<kPlaneInit>(a));
+        ADJ_RC(plane_init(a));
         PencilArgs<T> b = pencil_args();
         b.src = bf.gp;
         b.w = bf.lam;

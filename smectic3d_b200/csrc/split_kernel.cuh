@@ -122,10 +122,11 @@ struct ZrowCfg {
 enum ZrowMode : int {
   kZrowStep = 0,    // N(psi) alone
   kZrowGen = 1,     // also the penalties, psi out and the monitors (PassFlags)
-  kZrowReal = 2,    // slab[f] -> real_out[f] (field 0 with the monitors), no way back
+  kZrowReal = 2,    // slab[f] -> real_to[f] (field 0 with the monitors and psi out), no way back
   kZrowStress = 3,  // periodic advection: psi, L psi, grad psi to real space and (L psi) d_c psi forward
   kZrowMul = 4,     // real_in[f] real_in[3] (signed for the sine transform) forward -> slab[f]
   kZrowAdvN = 5,    // N(real_in[3]) - sum_c u_c real_in[c], the velocity from slab[c]; forward -> slab[0]
+  kZrowInit = 6,    // real psi (FP64) forward -> slab[0], N(psi) forward -> slab[1]
 };
 
 template <typename T>
@@ -139,6 +140,7 @@ struct ZrowArgs {
   int sign_axes;          // axis_sign of the real-space factors
   // kZrowGen, kZrowReal, kZrowStress
   int flags, plane0;      // first plane of the slab, rep * N + x
+  const double* psi_in;   // kZrowInit
   double* psi_out;
   const double* psi_old;
   double* red;            // per-CTA partial sums [plane][BLOCKS][3]
@@ -193,7 +195,15 @@ zrow_kernel(const __grid_constant__ ZrowArgs<T> a) {
     const int f = blockIdx.y;
     S::row_inverse(v, t, a.slab[f] + row_off, x, tw, false, typename S::Plain());
     if (f == 0) monitor();
-    S::real_store(v, t, a.real_to[f], ra, rb);
+    if (a.real_to[f]) S::real_store(v, t, a.real_to[f], ra, rb);
+  } else if constexpr (MODE == kZrowInit) {
+#pragma unroll
+    for (int s = 0; s < E; ++s) {
+      const int z = S::z_of(t, s);
+      v[s] = mk<T>(T(a.psi_in[ra + z]), T(a.psi_in[rb + z]));
+    }
+    if (blockIdx.y == 1) S::nonlin_penalties(v, t, x, a.pp, a.wall, a.lperp, a.kwall, ra, rb);
+    S::row_forward(v, t, a.slab[blockIdx.y] + row_off, x, tw, true, [] {}, typename S::Plain());
   } else if constexpr (MODE == kZrowMul) {
     // stress component S_c = (L psi) d_c psi of the Neumann Stokes solve
     // (cosFFT/comet/morphSurfK.cpp:760-770), signed for the sine transform
