@@ -1,0 +1,152 @@
+// Staged host copies (host_copy.cuh).
+#include "host_copy.cuh"
+
+#include <algorithm>
+#include <cstdint>
+#include <cstring>
+#include <mutex>
+#include <thread>
+
+namespace shb {
+namespace {
+
+constexpr int kWorkers = 6;               // memcpy threads; 6 x 8 GB/s is about the link rate
+constexpr size_t kChunk = size_t(1) << 19;  // per buffer, two buffers per worker: 6 MB pinned in all
+constexpr size_t kMin = size_t(4) << 20;    // below this the threads cost more than they save
+
+// One set of pinned buffers for the process: a copy that finds it taken (another
+// handle's copy on another thread) goes the plain way.
+struct Pool {
+  std::mutex use;    // held for the whole of a staged copy
+  std::mutex state;  // guards the members below
+  int handles = 0;
+  char* pinned = nullptr;
+};
+Pool& pool() {
+  static Pool p;
+  return p;
+}
+
+bool pageable(const void* host) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return at.type == cudaMemoryTypeUnregistered;
+}
+
+// worker w of n: chunks w, w + n, ... through its two buffers
+cudaError_t work(int w, int n, int device, char* pinned, char* host, char* dev, size_t bytes, bool to_device,
+                 cudaStream_t stream) {
+  cudaError_t e = cudaSetDevice(device);
+  cudaEvent_t done[2] = {nullptr, nullptr};
+  for (auto& ev : done)
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+  char* buf[2] = {pinned + size_t(2 * w) * kChunk, pinned + size_t(2 * w + 1) * kChunk};
+  const size_t chunks = (bytes + kChunk - 1) / kChunk;
+  size_t off[2] = {0, 0}, len[2] = {0, 0};  // chunk in flight in each buffer (len 0: none)
+  auto finish = [&](int b) {
+    if (e == cudaSuccess && len[b]) {
+      e = cudaEventSynchronize(done[b]);
+      if (e == cudaSuccess && !to_device) std::memcpy(host + off[b], buf[b], len[b]);
+    }
+    len[b] = 0;
+  };
+  int b = 0;
+  for (size_t c = w; c < chunks && e == cudaSuccess; c += n, b ^= 1) {
+    finish(b);
+    if (e != cudaSuccess) break;
+    off[b] = c * kChunk;
+    len[b] = std::min(kChunk, bytes - off[b]);
+    if (to_device) {
+      std::memcpy(buf[b], host + off[b], len[b]);
+      e = cudaMemcpyAsync(dev + off[b], buf[b], len[b], cudaMemcpyHostToDevice, stream);
+    } else {
+      e = cudaMemcpyAsync(buf[b], dev + off[b], len[b], cudaMemcpyDeviceToHost, stream);
+    }
+    if (e == cudaSuccess) e = cudaEventRecord(done[b], stream);
+  }
+  // the buffers are free for the next copy once these have passed
+  finish(b);
+  finish(b ^ 1);
+  if (e != cudaSuccess) cudaStreamSynchronize(stream);  // nothing still reads or writes the buffers
+  for (auto& ev : done)
+    if (ev) cudaEventDestroy(ev);
+  return e;
+}
+
+cudaError_t plain(void* dst, const void* src, size_t bytes, bool to_device, cudaStream_t stream) {
+  const cudaError_t e =
+      cudaMemcpyAsync(dst, src, bytes, to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, stream);
+  return e != cudaSuccess || to_device ? e : cudaStreamSynchronize(stream);
+}
+
+cudaError_t staged(void* dst, const void* src, size_t bytes, bool to_device, cudaStream_t stream) {
+  char* host = static_cast<char*>(to_device ? const_cast<void*>(src) : dst);
+  char* dev = static_cast<char*>(to_device ? dst : const_cast<void*>(src));
+  if (bytes < kMin || !pageable(host)) return plain(dst, src, bytes, to_device, stream);
+  Pool& p = pool();
+  std::unique_lock<std::mutex> lock(p.use, std::try_to_lock);
+  if (!lock.owns_lock()) return plain(dst, src, bytes, to_device, stream);
+  char* pinned;
+  {
+    std::lock_guard<std::mutex> g(p.state);
+    if (!p.pinned && p.handles > 0 && cudaHostAlloc(reinterpret_cast<void**>(&p.pinned), 2 * kWorkers * kChunk,
+                                                    cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      p.pinned = nullptr;
+    }
+    pinned = p.pinned;
+  }
+  if (!pinned) return plain(dst, src, bytes, to_device, stream);
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  std::thread th[kWorkers];
+  cudaError_t r[kWorkers];
+  bool run[kWorkers];
+  for (int w = 1; w < kWorkers; ++w) {
+    r[w] = cudaSuccess;
+    run[w] = true;
+    try {
+      th[w] = std::thread([&, w] { r[w] = work(w, kWorkers, device, pinned, host, dev, bytes, to_device, stream); });
+    } catch (...) {  // no thread to be had: its chunks follow on this one
+      run[w] = false;
+    }
+  }
+  e = work(0, kWorkers, device, pinned, host, dev, bytes, to_device, stream);
+  for (int w = 1; w < kWorkers; ++w) {
+    if (run[w]) th[w].join();
+    else r[w] = work(w, kWorkers, device, pinned, host, dev, bytes, to_device, stream);
+    if (e == cudaSuccess) e = r[w];
+  }
+  return e;
+}
+
+}  // namespace
+
+cudaError_t copy_to_device(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
+  return staged(dst, src, bytes, true, stream);
+}
+cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
+  return staged(dst, src, bytes, false, stream);
+}
+
+void host_copy_retain() {
+  Pool& p = pool();
+  std::lock_guard<std::mutex> g(p.state);
+  ++p.handles;
+}
+void host_copy_release() {
+  Pool& p = pool();
+  // a copy in flight belongs to a handle that still exists, so the buffers are idle
+  // when the count reaches 0
+  std::lock_guard<std::mutex> g(p.state);
+  if (--p.handles == 0 && p.pinned) {
+    cudaFreeHost(p.pinned);
+    p.pinned = nullptr;
+  }
+}
+
+}  // namespace shb

@@ -303,11 +303,11 @@ int sh_set_psi(sh_handle* h, const double* host_psi, int layout) {
   SolverBase* s = h->s;
   const size_t bytes = s->n3() * s->p.batch * sizeof(double);
   if (layout == SH_LAYOUT_DENSE) {
-    API_CUDA(h, cudaMemcpyAsync(s->d_psi, host_psi, bytes, cudaMemcpyHostToDevice, s->stream));
+    API_CUDA(h, copy_to_device(s->d_psi, host_psi, bytes, s->stream));
   } else {
     std::vector<double> tmp(s->n3() * s->p.batch);
     to_dense(host_psi, tmp.data(), s->p.n, s->p.batch, layout);
-    API_CUDA(h, cudaMemcpyAsync(s->d_psi, tmp.data(), bytes, cudaMemcpyHostToDevice, s->stream));
+    API_CUDA(h, copy_to_device(s->d_psi, tmp.data(), bytes, s->stream));
     API_CUDA(h, cudaStreamSynchronize(s->stream));
   }
   return sh_set_psi_device(h, s->d_psi);
@@ -336,12 +336,10 @@ int sh_get_psi(sh_handle* h, double* host_psi, int layout) {
   if (rc) return rc;
   const size_t bytes = s->n3() * s->p.batch * sizeof(double);
   if (layout == SH_LAYOUT_DENSE) {
-    API_CUDA(h, cudaMemcpyAsync(host_psi, s->d_psi, bytes, cudaMemcpyDeviceToHost, s->stream));
-    API_CUDA(h, cudaStreamSynchronize(s->stream));
+    API_CUDA(h, copy_to_host(host_psi, s->d_psi, bytes, s->stream));
   } else {
     std::vector<double> tmp(s->n3() * s->p.batch);
-    API_CUDA(h, cudaMemcpyAsync(tmp.data(), s->d_psi, bytes, cudaMemcpyDeviceToHost, s->stream));
-    API_CUDA(h, cudaStreamSynchronize(s->stream));
+    API_CUDA(h, copy_to_host(tmp.data(), s->d_psi, bytes, s->stream));
     from_dense(tmp.data(), host_psi, s->p.n, s->p.batch, layout);
   }
   return SH_OK;
@@ -370,8 +368,7 @@ int sh_local_amplitude(sh_handle* h, int nw, double* out) {
                                                                       lam * lam * lam);
   API_CUDA(h, cudaGetLastError());
   s->launches += 4;
-  API_CUDA(h, cudaMemcpyAsync(out, s->d_amp[1], bytes, cudaMemcpyDeviceToHost, s->stream));
-  API_CUDA(h, cudaStreamSynchronize(s->stream));
+  API_CUDA(h, copy_to_host(out, s->d_amp[1], bytes, s->stream));
   return SH_OK;
 }
 

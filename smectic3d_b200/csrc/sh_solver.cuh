@@ -10,6 +10,7 @@
 
 #include "../../include/smectic_b200.h"
 #include "flat_kernel.cuh"
+#include "host_copy.cuh"
 #include "pencil_kernel.cuh"
 #include "plane_kernel.cuh"
 #include "split_kernel.cuh"
@@ -100,8 +101,10 @@ struct SolverBase {
   // SH_ETIMEOUT.  Never set otherwise.
   int drop_exchange = 0;
 
+  SolverBase() { host_copy_retain(); }
   virtual ~SolverBase() {
     if (stream) cudaStreamSynchronize(stream);
+    host_copy_release();
     cudaFree(d_flag);
     cudaFree(d_psi);
     cudaFree(d_stash);
@@ -1176,8 +1179,7 @@ struct Solver final : SolverBase {
       to_double_kernel<T><<<4 * 148, 256, 0, stream>>>(R[5 + c], d_psi, (long long)nr);
       SHB_CUDA(cudaGetLastError());
       ++launches;
-      SHB_CUDA(cudaMemcpyAsync(outs[c], d_psi, nr * sizeof(double), cudaMemcpyDeviceToHost, stream));
-      SHB_CUDA(cudaStreamSynchronize(stream));
+      SHB_CUDA(copy_to_host(outs[c], d_psi, nr * sizeof(double), stream));
     }
     psi0_valid = false;  // d_psi was used as scratch
     return SH_OK;
@@ -1257,12 +1259,12 @@ struct Solver final : SolverBase {
     transpose_kernel<T><<<dim3(FP / 16, N / 16, p.batch), dim3(16, 16), 0, stream>>>(W, wt.p, N, FP);
     SHB_CUDA(cudaGetLastError());
     ++launches;
-    SHB_CUDA(cudaMemcpyAsync(h, wt.p, fb, cudaMemcpyDeviceToHost, stream));
-    SHB_CUDA(cudaMemcpyAsync(h + fb, P, fb, cudaMemcpyDeviceToHost, stream));
-    SHB_CUDA(cudaMemcpyAsync(h + 2 * fb, Nt, fb, cudaMemcpyDeviceToHost, stream));
+    SHB_CUDA(copy_to_host(h, wt.p, fb, stream));
+    SHB_CUDA(copy_to_host(h + fb, P, fb, stream));
+    SHB_CUDA(copy_to_host(h + 2 * fb, Nt, fb, stream));
     if (p.advection) {
-      SHB_CUDA(cudaMemcpyAsync(h + 3 * fb, Px, fb, cudaMemcpyDeviceToHost, stream));
-      SHB_CUDA(cudaMemcpyAsync(h + 4 * fb, PSH, fb, cudaMemcpyDeviceToHost, stream));
+      SHB_CUDA(copy_to_host(h + 3 * fb, Px, fb, stream));
+      SHB_CUDA(copy_to_host(h + 4 * fb, PSH, fb, stream));
     }
     SHB_CUDA(cudaStreamSynchronize(stream));
     return SH_OK;
@@ -1273,15 +1275,15 @@ struct Solver final : SolverBase {
     const char* h = static_cast<const char*>(host);
     DeviceScratch<cplx<T>> wt;
     SHB_CUDA(dev_malloc(&wt.p, fb));
-    SHB_CUDA(cudaMemcpyAsync(wt.p, h, fb, cudaMemcpyHostToDevice, stream));
+    SHB_CUDA(copy_to_device(wt.p, h, fb, stream));
     transpose_kernel<T><<<dim3(N / 16, FP / 16, p.batch), dim3(16, 16), 0, stream>>>(wt.p, W, FP, N);
     SHB_CUDA(cudaGetLastError());
     ++launches;
-    SHB_CUDA(cudaMemcpyAsync(P, h + fb, fb, cudaMemcpyHostToDevice, stream));
-    SHB_CUDA(cudaMemcpyAsync(Nt, h + 2 * fb, fb, cudaMemcpyHostToDevice, stream));
+    SHB_CUDA(copy_to_device(P, h + fb, fb, stream));
+    SHB_CUDA(copy_to_device(Nt, h + 2 * fb, fb, stream));
     if (p.advection) {
-      SHB_CUDA(cudaMemcpyAsync(Px, h + 3 * fb, fb, cudaMemcpyHostToDevice, stream));
-      SHB_CUDA(cudaMemcpyAsync(PSH, h + 4 * fb, fb, cudaMemcpyHostToDevice, stream));
+      SHB_CUDA(copy_to_device(Px, h + 3 * fb, fb, stream));
+      SHB_CUDA(copy_to_device(PSH, h + 4 * fb, fb, stream));
     }
     SHB_CUDA(cudaStreamSynchronize(stream));
     ready = true;
@@ -1364,7 +1366,7 @@ struct Solver final : SolverBase {
       bf.k = K;
     }
     const size_t fb = fe * sizeof(cplx<T>);
-    ADJ_CUDA(cudaMemcpyAsync(d_psi, psi0, nr * sizeof(double), cudaMemcpyHostToDevice, stream));
+    ADJ_CUDA(copy_to_device(d_psi, psi0, nr * sizeof(double), stream));
     ADJ_RC(init_from_psi());
     for (int sg = 0; sg < nseg; ++sg) {
       cplx<T>* c = bf.ck + size_t(sg) * 3 * fe;
@@ -1454,7 +1456,7 @@ struct Solver final : SolverBase {
       ADJ_CUDA(cudaMemcpyAsync(bf.fin + fe, P, fb, cudaMemcpyDeviceToDevice, stream));
       ADJ_CUDA(cudaMemcpyAsync(bf.fin + 2 * fe, Nt, fb, cudaMemcpyDeviceToDevice, stream));
       // ---- lambda^T -> lambdahat^T and the partial of mu^T = B lambda^T
-      ADJ_CUDA(cudaMemcpyAsync(d_psi, dl_dpsi_t, nr * sizeof(double), cudaMemcpyHostToDevice, stream));
+      ADJ_CUDA(copy_to_device(d_psi, dl_dpsi_t, nr * sizeof(double), stream));
       {
         PlaneArgs<T> a = plane_args();
         a.psi_in = d_psi;
@@ -1530,7 +1532,7 @@ struct Solver final : SolverBase {
       }
       std::vector<double> acc(size_t(p.batch) * 4);
       ADJ_CUDA(cudaMemcpyAsync(acc.data(), bf.acc, acc.size() * sizeof(double), cudaMemcpyDeviceToHost, stream));
-      ADJ_CUDA(cudaMemcpyAsync(g_psi0, d_psi, nr * sizeof(double), cudaMemcpyDeviceToHost, stream));
+      ADJ_CUDA(copy_to_host(g_psi0, d_psi, nr * sizeof(double), stream));
       // back to the state the forward sweep ended in
       ADJ_CUDA(cudaMemcpyAsync(W, bf.fin, fb, cudaMemcpyDeviceToDevice, stream));
       ADJ_CUDA(cudaMemcpyAsync(P, bf.fin + fe, fb, cudaMemcpyDeviceToDevice, stream));

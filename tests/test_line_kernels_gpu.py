@@ -117,3 +117,31 @@ def test_checkpoint_file_keeps_w_by_line(boundary):
         got = np.frombuffer(blob, np.float64, n * n * n, head).reshape(n, n // 2, n, 2)  # [ky][kz / 2][kx][kz % 2]
         want = w.reshape(n, n, n // 2, 2).transpose(1, 2, 0, 3)
     assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("n,b", [(64, 1), (64, 2), (32, 17), (128, 1)])
+def test_host_arrays_cross_unchanged(n, b):
+    """Pageable arrays below, at and above the size that is staged by threads (4 MB),
+    with a ragged last chunk: psi^0 comes back as it went in, also when two handles
+    copy at the same time from two threads (one of them then goes the plain way)."""
+    import threading
+
+    psi = np.random.default_rng(n + b).uniform(-1, 1, size=(b, n, n, n))
+    p = S.Params(n=n, batch=b, precision="fp64")
+    bad = []
+
+    def loop(shift):
+        with S.Solver(p) as s:
+            for k in range(5):
+                a = (psi + shift + k).reshape(s.shape)
+                s.set_psi(a)
+                if not np.array_equal(s.get_psi(), a):
+                    bad.append((shift, k))
+
+    loop(0)
+    threads = [threading.Thread(target=loop, args=(10 * i,)) for i in range(1, 3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
