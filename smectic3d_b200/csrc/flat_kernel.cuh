@@ -22,8 +22,8 @@ struct FlatCfg {
   static constexpr int THREADS = (N / 2) * G;
   static constexpr int FP = DCT ? N * (N / 2) : N * (N / 2 + 1);
   // padded row pair: room for the warp exchange, and the lines of a half-warp on
-  // different banks (G = 4: four lines, G = 8: two)
-  static constexpr int LS = N + (G == 4 ? 4 : 8);
+  // different banks (G = 4: four lines, a stride of 4 mod 16; G = 8: two, 8 mod 16)
+  static constexpr int LS = (warp_line<N>() + 15) / 16 * 16 + (G == 4 ? 4 : 8);
   static constexpr size_t ROWS = size_t(N / 2) * LS, COLS = size_t(N) * (N / 2);
   static constexpr size_t PK_OFF = (ROWS > COLS ? ROWS : COLS) * sizeof(cplx<T>);
   // the packed kz = 0 / N/2 column of the periodic box

@@ -156,18 +156,28 @@ template <typename T, int TK>
 struct TileExchange {
   cplx<T>* base;  // tile + c
   __device__ __forceinline__ void sync() const { __syncthreads(); }
+  template <int R>
   __device__ __forceinline__ void store(int p, cplx<T> v) const { base[p * TK] = v; }
+  template <int R>
   __device__ __forceinline__ cplx<T> load(int p) const { return base[p * TK]; }
 };
-// Exchange inside a warp: the G threads of a line are consecutive lanes, the
-// line is padded by one slot every RA (forward) or RB (inverse) elements.
+// Exchange inside a warp: the G threads of a line are consecutive lanes.  Every R
+// elements, R the radix that stores them, are followed by one slot of padding: the
+// stores of neighbouring threads are R + 1 apart and their loads consecutive, which
+// with the line strides of the kernels is free of bank conflicts both ways (a fixed
+// 16 made the inverse stores of the 64-point lines four-way).
 template <typename T>
 struct WarpExchange {
   cplx<T>* line;
   __device__ __forceinline__ void sync() const { __syncwarp(); }
-  __device__ __forceinline__ void store(int p, cplx<T> v) const { line[p + (p >> 4)] = v; }
-  __device__ __forceinline__ cplx<T> load(int p) const { return line[p + (p >> 4)]; }
+  template <int R>
+  __device__ __forceinline__ void store(int p, cplx<T> v) const { line[p + p / R] = v; }
+  template <int R>
+  __device__ __forceinline__ cplx<T> load(int p) const { return line[p + p / R]; }
 };
+// slots of such a line
+template <int N>
+__host__ __device__ constexpr int warp_line() { return N + N / LinePlan<N>::RB; }
 
 template <typename T, int N>
 struct LineFFT {
@@ -184,10 +194,10 @@ struct LineFFT {
 #pragma unroll
     for (int a = 0; a < NA; ++a)
 #pragma unroll
-      for (int q = 0; q < RA; ++q) x.store(I::ja(t, a) * RA + q, v[a * RA + q]);
+      for (int q = 0; q < RA; ++q) x.template store<RA>(I::ja(t, a) * RA + q, v[a * RA + q]);
     x.sync();
 #pragma unroll
-    for (int s = 0; s < E; ++s) v[s] = x.load(I::b_elem(t, s));
+    for (int s = 0; s < E; ++s) v[s] = x.template load<RA>(I::b_elem(t, s));
 #pragma unroll
     for (int s = 0; s < E; s += 2) {
       cplx<T> w0, w1;
@@ -208,10 +218,10 @@ struct LineFFT {
 #pragma unroll
     for (int b = 0; b < NB; ++b)
 #pragma unroll
-      for (int q = 0; q < RB; ++q) x.store(I::jb(t, b) * RB + q, v[b * RB + q]);
+      for (int q = 0; q < RB; ++q) x.template store<RB>(I::jb(t, b) * RB + q, v[b * RB + q]);
     x.sync();
 #pragma unroll
-    for (int s = 0; s < E; ++s) v[s] = x.load(I::a_elem(t, s));
+    for (int s = 0; s < E; ++s) v[s] = x.template load<RB>(I::a_elem(t, s));
 #pragma unroll
     for (int s = 0; s < E; s += 2) {
       cplx<T> w0, w1;

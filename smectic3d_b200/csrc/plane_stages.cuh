@@ -305,7 +305,7 @@ struct PlaneStages {
     if (pp.w_mid != 0.0) {
       x.sync();
 #pragma unroll
-      for (int s = 0; s < E; ++s) x.store(z_of(t, s), v[s]);
+      for (int s = 0; s < E; ++s) x.template store<16>(z_of(t, s), v[s]);
       x.sync();
     }
     const T* lpa = kwall > 0 ? lperp + (ra / N) * kwall : nullptr;
@@ -316,7 +316,7 @@ struct PlaneStages {
       const cplx<T> q = v[s];
       cplx<T> o = mk<T>(nonlin_eval<T>(q.x, beta, gamma, pp.nonlin), nonlin_eval<T>(q.y, beta, gamma, pp.nonlin));
       if (pp.w_mid != 0.0 && z == N / 2) {
-        const cplx<T> lo = x.load(z - 1), hi = x.load(z + 1);
+        const cplx<T> lo = x.template load<16>(z - 1), hi = x.template load<16>(z + 1);
         const T cw = T(2.0 * pp.w_mid * pp.inv_dz2);
         o.x += cw * (lo.x - T(2) * q.x + hi.x);
         o.y += cw * (lo.y - T(2) * q.y + hi.y);

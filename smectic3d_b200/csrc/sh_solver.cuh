@@ -174,6 +174,7 @@ struct Solver final : SolverBase {
   // null where the plane pass is one kernel
   cplx<T>* slab = nullptr;
   int slab_planes = 0;
+  char* tables = nullptr;  // one allocation for the tables below (tw, lt, q, qd, qs, qds)
   cplx<T>* tw = nullptr;  // [forward | inverse | quarter-wave] twiddle table
   cplx<T>* lt = nullptr;  // line tables (LineTab)
   // Stokes advection (periodic): partials of i q_x psihat and opSH psihat, the
@@ -233,12 +234,7 @@ struct Solver final : SolverBase {
     cudaFree(P);
     cudaFree(Nt);
     cudaFree(slab);
-    cudaFree(tw);
-    cudaFree(lt);
-    cudaFree(q);
-    cudaFree(qd);
-    cudaFree(qs);
-    cudaFree(qds);
+    cudaFree(tables);
     cudaFree(Px);
     cudaFree(PSH);
     for (auto* p3 : S3) cudaFree(p3);
@@ -364,12 +360,6 @@ struct Solver final : SolverBase {
         SHB_CUDA(cudaMemcpy(d_wall, hw.data(), kwall * sizeof(T), cudaMemcpyHostToDevice));
       }
     }
-    SHB_CUDA(dev_malloc(&tw, tw_total<N>() * sizeof(cplx<T>)));
-    SHB_CUDA(dev_malloc(&q, N * sizeof(T)));
-    SHB_CUDA(dev_malloc(&qd, N * sizeof(double)));
-    SHB_CUDA(dev_malloc(&lt, LineTab<N>::total * sizeof(cplx<T>)));
-    SHB_CUDA(dev_malloc(&qs, N * sizeof(T)));
-    SHB_CUDA(dev_malloc(&qds, N * sizeof(double)));
     SHB_CUDA(dev_malloc(&d_red_plane, size_t(p.batch) * N * std::max(CL, kSplit ? ZC::BLOCKS : 1) * 3 * sizeof(double)));
     SHB_CUDA(dev_malloc(&d_red_spec, size_t(p.batch) * QC::TILES * sizeof(double)));
     std::vector<cplx<T>> htw;
@@ -385,9 +375,6 @@ struct Solver final : SolverBase {
       for (int i = 0; i < N; ++i) hqd[i] = M_PI * i / (p.dx * N);
     }
     for (int i = 0; i < N; ++i) hq[i] = T(hqd[i]);
-    SHB_CUDA(cudaMemcpy(qd, hqd.data(), N * sizeof(double), cudaMemcpyHostToDevice));
-    SHB_CUDA(cudaMemcpy(tw, htw.data(), htw.size() * sizeof(cplx<T>), cudaMemcpyHostToDevice));
-    SHB_CUDA(cudaMemcpy(q, hq.data(), N * sizeof(T), cudaMemcpyHostToDevice));
     std::vector<cplx<T>> hlt;
     host_line_tables<T, N>(hlt);
     std::vector<T> hqs(N);
@@ -398,9 +385,25 @@ struct Solver final : SolverBase {
         hqs[t * QC::E + s] = hq[k];
         hqds[t * QC::E + s] = hqd[k];
       }
-    SHB_CUDA(cudaMemcpy(lt, hlt.data(), hlt.size() * sizeof(cplx<T>), cudaMemcpyHostToDevice));
-    SHB_CUDA(cudaMemcpy(qs, hqs.data(), N * sizeof(T), cudaMemcpyHostToDevice));
-    SHB_CUDA(cudaMemcpy(qds, hqds.data(), N * sizeof(double), cudaMemcpyHostToDevice));
+    // all tables in one allocation and one copy, each 256-byte aligned
+    std::vector<char> img;
+    auto put = [&](const void* src, size_t bytes) {
+      const size_t at = align_up(img.size(), 256);
+      img.resize(at + bytes);
+      std::memcpy(img.data() + at, src, bytes);
+      return at;
+    };
+    const size_t o_tw = put(htw.data(), htw.size() * sizeof(cplx<T>)), o_lt = put(hlt.data(), hlt.size() * sizeof(cplx<T>));
+    const size_t o_q = put(hq.data(), N * sizeof(T)), o_qd = put(hqd.data(), N * sizeof(double));
+    const size_t o_qs = put(hqs.data(), N * sizeof(T)), o_qds = put(hqds.data(), N * sizeof(double));
+    SHB_CUDA(dev_malloc(&tables, img.size()));
+    SHB_CUDA(cudaMemcpy(tables, img.data(), img.size(), cudaMemcpyHostToDevice));
+    tw = reinterpret_cast<cplx<T>*>(tables + o_tw);
+    lt = reinterpret_cast<cplx<T>*>(tables + o_lt);
+    q = reinterpret_cast<T*>(tables + o_q);
+    qd = reinterpret_cast<double*>(tables + o_qd);
+    qs = reinterpret_cast<T*>(tables + o_qs);
+    qds = reinterpret_cast<double*>(tables + o_qds);
     int rc;
     if ((rc = set_attrs(plane_fn<kPlaneStep>(), kPlaneSmem, true))) return rc;
     if ((rc = set_attrs(plane_fn<kPlaneInit>(), kPlaneSmem, true))) return rc;

@@ -104,7 +104,7 @@ struct ZrowCfg {
   static constexpr int BLOCKS = N / 2 / LINES;  // CTAs per plane
   static constexpr int SP = N * (N / 2);
   // padded line; the + 8 puts the two lines of a half-warp on different banks
-  static constexpr int LS = N + N / 16 + 8;
+  static constexpr int LS = warp_line<N>() + 8;
   static constexpr size_t RED_OFF = size_t(LINES) * LS * sizeof(cplx<T>);
   static constexpr size_t KEEP_OFF = RED_OFF + 16 * sizeof(double);  // one value per slot and thread kept aside
   static constexpr size_t smem(int mode) {
