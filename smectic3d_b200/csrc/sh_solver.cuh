@@ -119,6 +119,7 @@ struct SolverBase {
     for (auto& e : prof_ev)
       if (e) cudaEventDestroy(e);
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
+    if (graph_one) cudaGraphExecDestroy(graph_one);
     if (stream) cudaStreamDestroy(stream);
   }
   size_t n3() const { return size_t(p.n) * p.n * p.n; }
@@ -133,6 +134,7 @@ struct SolverBase {
   // bookkeeping is needed: no energy trace, L1 monitor, profiling or history)
   static constexpr int kGraphChunk = 16;
   cudaGraphExec_t graph_exec = nullptr;
+  cudaGraphExec_t graph_one = nullptr;  // one step, for steps of many launches (Solver::many_launches)
   bool use_graphs = true;
   virtual int psi_to_dpsi() = 0;       // current psi -> d_psi
   virtual int energy_now(double* host) = 0;
@@ -851,9 +853,18 @@ struct Solver final : SolverBase {
     return SH_OK;
   }
 
-  // capture kGraphChunk steps once (nothing runs; the steps counter is restored)
-  int build_graph() override {
-    if (graph_exec || !graph_eligible()) return SH_OK;
+  // A step that goes slab by slab is 21 to 60 launches, and outside a graph each
+  // costs the GPU about 3 us between kernels (advected 256^3 FP32: 930 us per step
+  // launched one by one, 824 replayed): its steps outside the kGraphChunk graph
+  // replay a graph of one step.
+  bool split_advected() const { return kSplit && slab != nullptr; }
+  bool many_launches() const {
+    if constexpr (kSplit) return slab != nullptr && (long long)p.batch * N > slab_planes && !blocked();
+    else return false;
+  }
+
+  // capture ``n`` plain steps (nothing runs; the steps counter is restored)
+  int capture(int n, cudaGraphExec_t* exec, long long* count) {
     cudaGraph_t g;
     const long long s0 = steps, l0 = launches;
     // the graph holds plain steps only: the L1 monitor's steps run outside it
@@ -864,25 +875,59 @@ struct Solver final : SolverBase {
     if (blocked()) {
       for (int r0 = 0; r0 < p.batch && !rc; r0 += p.replica_block) {
         const int gsz = r0 + p.replica_block <= p.batch ? p.replica_block : p.batch - r0;
-        rc = step_window(r0, gsz, kGraphChunk);
+        rc = step_window(r0, gsz, n);
       }
-      steps += kGraphChunk;
-      hist_pos += kGraphChunk;
+      steps += n;
+      hist_pos += n;
     } else {
-      rc = step_direct(kGraphChunk);
+      rc = step_direct(n);
     }
     cudaError_t e = cudaStreamEndCapture(stream, &g);
     p.l1_interval = li;
     steps = s0;
-    hist_pos -= kGraphChunk;
-    graph_launches = launches - l0;
+    hist_pos -= n;
+    *count = launches - l0;
     launches = l0;
     if (rc) return rc;
     SHB_CUDA(e);
-    e = cudaGraphInstantiate(&graph_exec, g, 0);
+    e = cudaGraphInstantiate(exec, g, 0);
     cudaGraphDestroy(g);
     SHB_CUDA(e);
     return SH_OK;
+  }
+  int build_graph() override {
+    int rc;
+    if (!graph_eligible()) return SH_OK;
+    if (many_launches() && !graph_one && (rc = capture(1, &graph_one, &one_launches))) return rc;
+    if (graph_exec) return SH_OK;
+    return capture(kGraphChunk, &graph_exec, &graph_launches);
+  }
+
+  // steps outside the kGraphChunk graph
+  int step_few(int n) {
+    if (!many_launches() || !graph_eligible()) return step_direct(n);
+    int rc;
+    const int li = p.l1_interval;
+    for (; n > 0; --n) {
+      const long long c = steps + 1;
+      if (li > 0 && (c % li == 0 || (c + 1) % li == 0)) {
+        if ((rc = step_direct(1))) return rc;
+        continue;
+      }
+      if (!graph_one && (rc = capture(1, &graph_one, &one_launches))) return rc;
+      SHB_CUDA(cudaGraphLaunch(graph_one, stream));
+      ++steps;
+      launches += one_launches;
+      replayed();
+    }
+    return SH_OK;
+  }
+  // what adv_nonlinear notes when its kernels run outside a graph
+  void replayed() {
+    if (!p.advection) return;
+    real_fields_current = true;
+    lpsi_current = !split_advected() || DCT;
+    u_real_current = false;
   }
 
   int step_async(int n) override {
@@ -895,8 +940,9 @@ struct Solver final : SolverBase {
           SHB_CUDA(cudaGraphLaunch(graph_exec, stream));
           steps += kGraphChunk;
           launches += graph_launches;
+          replayed();
         }
-        return step_direct(n - chunks * kGraphChunk);
+        return step_few(n - chunks * kGraphChunk);
       }
       // L1 monitor on (the reference's loop): replay the graph over the chunks
       // that hold no monitored step, take the steps around each one directly
@@ -905,17 +951,18 @@ struct Solver final : SolverBase {
           SHB_CUDA(cudaGraphLaunch(graph_exec, stream));
           steps += kGraphChunk;
           launches += graph_launches;
+          replayed();
           n -= kGraphChunk;
         } else {
-          if ((rc = step_direct(1))) return rc;
+          if ((rc = step_few(1))) return rc;
           --n;
         }
       }
       return SH_OK;
     }
-    return step_direct(n);
+    return step_few(n);
   }
-  long long graph_launches = 0;
+  long long graph_launches = 0, one_launches = 0;
 
   int step_direct(int n) {
     int rc;

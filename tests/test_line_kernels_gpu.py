@@ -145,3 +145,23 @@ def test_host_arrays_cross_unchanged(n, b):
     for t in threads:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("n,boundary", [(64, "periodic"), (256, "periodic"), (256, "neumann")])
+def test_advected_replays_equal_direct_steps(n, boundary):
+    """Steps replayed from the graphs (one step at 256^3, 16 steps) leave the state,
+    the velocity and the surface pass of steps launched one by one."""
+    psi = _psi(n, 9, 0.9)
+    kw = dict(n=n, boundary=boundary, precision="fp32", advection=True, dt=0.02)
+    with S.Solver(S.Params(**kw)) as a, S.Solver(S.Params(energy_trace=True, **kw)) as b:  # a trace runs outside graphs
+        for s in (a, b):
+            s.set_psi(psi)
+        for k in (3, 16, 1):
+            for s in (a, b):
+                s.step(k)
+            assert np.array_equal(a.get_psi(), b.get_psi()), k
+            for u, v in zip(a.velocity(), b.velocity()):
+                assert np.array_equal(u, v), k
+            if boundary == "periodic":
+                for u, v in zip(a.surface_step(), b.surface_step()):
+                    assert np.array_equal(u, v, equal_nan=True), k
