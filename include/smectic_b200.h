@@ -66,8 +66,10 @@ typedef struct sh_params {
   int precision;     /* SH_FP64 / SH_FP32                                    */
   int l1_interval;   /* steps between L1 evaluations (pf3d.cpp:489: 100); 0 = off */
   int energy_trace;  /* 1: record the energy of every new state              */
-  int variant;       /* plane-pass cluster size (0 = default; built: 1, 2 at 64^3;
-                        1, 2, 4 at 128^3; 4, 8, 16 at 256^3; 16 at 512^3)     */
+  int variant;       /* cluster size of the clustered plane pass (0 = default; built: 1, 2
+                        at 64^3; 1, 2, 4 at 128^3; 4, 8, 16 at 256^3; 16 at 512^3).  1 is
+                        the one-CTA form; plain and advected steps at 256^3 and 512^3 run
+                        one axis at a time instead and do not depend on it */
   double dx, dt, eps, beta, gamma, alpha, q0, eta, rho;
   double w_mid;      /* pinning penalty weight (periodicFFT/pf3dMorph.cpp:102) */
   double sub_sigma;  /* substrate penalty sigma (cosFFT/comet/cosNoAdvMorph.cpp:67-74) */
@@ -233,7 +235,9 @@ int sh_host_free(void* p);
  * the summed device milliseconds of the pencil (x) and plane (y,z) passes. */
 int sh_profile_steps(sh_handle* h, int nsteps, double* ms_pencil, double* ms_plane);
 
-/* Residency of the two step kernels on the handle's GPU, written to out[7]:
+/* Residency of the pencil kernel and of the plane kernel of the handle's
+ * cluster size on the handle's GPU (the step's own plane kernel up to 128^3; at
+ * 256^3 and 512^3 the kernel of the passes that still run clustered), to out[7]:
  *   out[0] plane-pass CTAs per SM, out[1] plane clusters resident at once,
  *   out[2] plane cluster size (CTAs), out[3] plane CTAs in one pass,
  *   out[4] pencil-pass CTAs per SM, out[5] pencil CTAs in one pass,

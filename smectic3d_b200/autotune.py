@@ -3,7 +3,8 @@
 Each built shape offers a few cluster sizes for the plane pass (``variant``):
 - CL = 1 and 2 at 64^3;
 - CL = 1, 2 and 4 at 128^3;
-- CL = 4, 8 and 16 at 256^3.
+- CL = 4, 8 and 16 at 256^3 (only for the passes that run clustered there; the
+  steps themselves go one axis at a time and time alike).
 
 Batched runs of small grids also choose ``replica_block``: how many replicas
 advance together, 16 steps at a time, while their state stays in the 126 MB L2

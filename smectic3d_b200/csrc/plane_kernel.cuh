@@ -21,6 +21,10 @@
 // Neumann transforms are REDFT01 / REDFT10 computed as one complex N-point FFT
 // with the even/odd permutation and quarter-wave twiddles (Makhoul), applied to
 // two real sequences at once (the transform is linear).
+//
+// This form serves 16^2 planes, the cluster sizes a handle asks for, and at 256^2
+// and 512^2 the modes that split_kernel.cuh does not have; flat_kernel.cuh takes
+// planes of 32^2 to 128^2 with one CTA (64 x 64^3 FP32 step pass 85 -> 54 us).
 #pragma once
 #include "sh_common.cuh"
 

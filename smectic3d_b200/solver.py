@@ -41,7 +41,7 @@ class Params:
     sub_sigma: float = 0.0
     sub_z0: float = 1e-4
     eps_per_replica: tuple | None = None
-    variant: int = 0                 # plane-pass cluster size (0 = default, -1 = autotune)
+    variant: int = 0                 # cluster size of the clustered plane pass (0 = default, -1 = autotune)
     curvature: str = "difference"    # Neumann curvature pass: "difference" (reference) | "spectral"
     replica_block: int = 0           # batched plain steps: replicas per L2-resident block (0 = off)
     pencil_tile: int = 0             # lines per pencil CTA (0 = default; 8, 16, 32 at 64^3 and 128^3)
@@ -155,7 +155,7 @@ class Solver:
         return a.value, b.value
 
     def residency(self) -> dict:
-        """CTAs per SM and waves of the two step kernels on this GPU."""
+        """CTAs per SM and waves of the pencil kernel and the (one-CTA or clustered) plane kernel."""
         o = (C.c_int * 7)()
         self._chk(self.lib.sh_residency(self.h, o))
         plane_res = o[1] * o[2]
