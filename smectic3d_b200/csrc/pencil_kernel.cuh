@@ -241,7 +241,7 @@ __device__ __forceinline__ double rcp2(double x) {
 __device__ __forceinline__ double2 rcp2(double2 x) { return make_double2(rcp2(x.x), rcp2(x.y)); }
 
 // What bounds it: Neumann 256^3 FP32 moves 268 MB (41 us at the measured copy
-// rate) in 63 us; 22.4 M warp instructions (35 % of the issue slots), 2.2 M
+// rate) in 57 us; 24.0 M warp instructions (41 % of the issue slots), 2.1 M
 // shared-memory wavefronts; the waits are the HBM latency of the line loads and of
 // W.  The 16-values-per-thread form it replaces staged tiles in shared memory and
 // paired k with N - k by shuffles: 42 M instructions, 7.5 M wavefronts, 76 us.

@@ -153,7 +153,9 @@ struct ZrowArgs {
 };
 
 // The three passes against the clustered kernel: Neumann 256^3 FP32 113 -> 80 us,
-// periodic 94 -> 71, Neumann 256^3 FP64 262 -> 183, 512^3 FP64 5408 -> 1578.
+// periodic 94 -> 71, Neumann 256^3 FP64 262 -> 183, 512^3 FP64 5408 -> 1578.  The z
+// pass is the longest (36 us Neumann 256^3 FP32): two transforms and the pointwise
+// work, 19.7 M warp instructions, issue slots 55 % busy.
 //
 // z transforms of LINES row pairs around the real-space work.  G consecutive
 // lanes own a line and exchange inside their warp: no block barrier, every warp
