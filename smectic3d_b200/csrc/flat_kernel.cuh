@@ -6,11 +6,13 @@
 // global memory; in the row stage the G lanes of a row pair are neighbours and
 // exchange inside their warp.  One buffer serves the column exchange, the row pairs
 // and the row exchanges (a row pair is its own scratch), so shared memory holds the
-// plane once.  Neumann rows are packed two by two (2 p, 2 p + 1) as in
-// plane_kernel.cuh, so FP32 results stay bit for bit those of that kernel.
+// plane once.  Rows are packed two by two (2 p, 2 p + 1) as in plane_kernel.cuh, one
+// after the other in the pair, so psi and the gradients of FP32 (and periodic FP64)
+// runs are bit for bit those of that kernel.  Pairs of rows p and p + N / 2, which a
+// periodic column holds in one thread and can store as 16 bytes, round every step
+// otherwise and gain nothing: 64 x 64^3 FP32 step 95.8 us, 93.2 with neighbours;
+// 128^3 FP64 27.7, 26.4; 128^3 FP32 15.1, 15.4.
 #pragma once
-#include <type_traits>
-
 #include "plane_stages.cuh"
 
 namespace shb {
@@ -49,7 +51,7 @@ flat_kernel(const __grid_constant__ PlaneLaunch<T> pl) {
   using Cfg = FlatCfg<T, N, DCT>;
   using S = PlaneStages<T, N, DCT>;
   using Ops = PlaneOps<T, N, 1, DCT>;
-  using Access = std::conditional_t<DCT, typename S::Planar, typename S::Plain>;
+  using Access = typename S::Planar;
   constexpr int E = Cfg::E, G = Cfg::G, LS = Cfg::LS, NC = N / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<T>* buf = reinterpret_cast<cplx<T>*>(smem_raw);
@@ -66,7 +68,7 @@ flat_kernel(const __grid_constant__ PlaneLaunch<T> pl) {
   const RowTables<T, N> rtw(a.lt, rt);
   const int x = blockIdx.x, rep = blockIdx.y;
   const size_t plane_off = (size_t(rep) * N + x) * Cfg::FP;
-  const int ya = DCT ? 2 * p : p, yb = DCT ? 2 * p + 1 : p + N / 2;
+  const int ya = 2 * p, yb = 2 * p + 1;
   const size_t ra = ((size_t(rep) * N + x) * N + ya) * N, rb = ((size_t(rep) * N + x) * N + yb) * N;
   cplx<T> v[E];
   grid_dependency_wait();
@@ -108,16 +110,14 @@ flat_kernel(const __grid_constant__ PlaneLaunch<T> pl) {
     }
     S::col_inverse(v, ct, cx, ctw, busy, false, [](int) { return cplx<T>(); });
     __syncthreads();  // every line has left the exchange
-    if constexpr (DCT) S::to_planar(v, ct, buf, c, LS);
-    else S::to_pairs(v, ct, buf + 2 * c, LS);
+    S::to_planar(v, ct, buf, c, LS);
     __syncthreads();
   };
   // rows on the A side -> partial spectrum
   auto rows_out = [&](cplx<T>* __restrict__ plane, bool busy) {
     S::row_forward(v, rt, row, rx, rtw, busy, [&] { rx.sync(); }, Access());
     __syncthreads();
-    if constexpr (DCT) S::from_planar(v, ct, buf, c, LS);
-    else S::from_pairs(v, ct, buf + 2 * c, LS);
+    S::from_planar(v, ct, buf, c, LS);
     S::col_forward(v, ct, cx, ctw, true, false, [](int, cplx<T>) {});
     if (DCT || c > 0) {
 #pragma unroll

@@ -3,12 +3,13 @@
 // (split_kernel.cuh).
 //
 // Between the stages a plane is kept as row pairs, which is what the z stage packs
-// into one complex line:
+// into one complex line.  In the split passes' slab:
 //   [p][2 c + h], p < N/2, rows real_pos(p) and real_pos(p + N/2)
 //   periodic: h = 0, 1: kz = c of either row (kz = 0 carries F0 + i FN)
 //   Neumann : z = 2 c + h, as (first row, second row)
 // A column thread ends with both rows of a pair in registers, so a pair of columns
-// moves as one 16-byte access (32 in FP64).
+// moves as one 16-byte access (32 in FP64).  The one-CTA pass keeps rows 2 p and
+// 2 p + 1, one after the other (Planar).
 #pragma once
 #include "line_fft.cuh"
 #include "plane_kernel.cuh"
@@ -125,8 +126,8 @@ struct PlaneStages {
     }
   }
 
-  // ---- row stage: a row pair [2 c + h] -> psi of the two rows on the A side.
-  // ``mul(k, value)``: spectral multiplier of a row's kz = k (identity for most)
+  // ---- row stage: a row pair -> psi of the two rows on the A side.  ``mul`` reads
+  // the pair's kz = k, in its layout and times its spectral multiplier
   template <class X, class Tab, class Mul>
   static __device__ __forceinline__ void row_inverse(cplx<T> (&v)[E], int t, const cplx<T>* row, const X& x,
                                                      const Tab& tw, bool first_sync, Mul mul) {
@@ -140,8 +141,7 @@ struct PlaneStages {
       for (int s = 0; s < E / 2; ++s) {
         const int k = I::c_low(s) ? I::c_elem(t, s) : N - I::c_elem(t, s);  // < N/2
         cplx<T> A, B;
-        ld2(row + 2 * k, A, B);
-        mul(k, A, B);
+        mul.load(k, row, A, B);
         cplx<T> zk = mk<T>(A.x - B.y, A.y + B.x), zm = mk<T>(A.x + B.y, B.x - A.y);
         if (s == 0 && t == 0) {
           zk = mk<T>(A.x, B.x);
@@ -178,20 +178,24 @@ struct PlaneStages {
           A = mk<T>(z.x, zm.x);
           B = mk<T>(z.y, zm.y);
         }
-        st2(row + 2 * k, A, B);
+        put.store(k, row, A, B);
       }
     }
   }
-  // row access of most passes: no multiplier, (first row, second row) interleaved
+  // row access of the split passes: no multiplier, (first row, second row) interleaved
   struct Plain {
     __device__ __forceinline__ cplx<T> operator()(int k, const cplx<T>* row) const { return row[k]; }
     __device__ __forceinline__ void operator()(int k, cplx<T>* row, cplx<T> z) const { row[k] = z; }
-    __device__ __forceinline__ void operator()(int, cplx<T>&, cplx<T>&) const {}
+    __device__ __forceinline__ void load(int k, const cplx<T>* row, cplx<T>& A, cplx<T>& B) const {
+      ld2(row + 2 * k, A, B);
+    }
+    __device__ __forceinline__ void store(int k, cplx<T>* row, cplx<T> A, cplx<T> B) const { st2(row + 2 * k, A, B); }
   };
   // d/dz of a periodic row when q is given: i q_z
   struct Dz {
     const T* q;
-    __device__ __forceinline__ void operator()(int k, cplx<T>& A, cplx<T>& B) const {
+    __device__ __forceinline__ void load(int k, const cplx<T>* row, cplx<T>& A, cplx<T>& B) const {
+      ld2(row + 2 * k, A, B);
       if (q) {
         // the kz = 0 slot holds the kz = 0 and N/2 columns, whose z derivatives vanish
         const T qz = k != 0 ? __ldg(&q[k]) : T(0);
@@ -200,7 +204,8 @@ struct PlaneStages {
       }
     }
   };
-  // Neumann rows one after the other: N values of the first row, then the second
+  // rows one after the other: N values (Neumann) or N / 2 complex values (periodic)
+  // of the first row, then the second
   struct Planar {
     __device__ __forceinline__ cplx<T> operator()(int k, const cplx<T>* row) const {
       const T* f = reinterpret_cast<const T*>(row);
@@ -211,7 +216,14 @@ struct PlaneStages {
       f[k] = z.x;
       f[N + k] = z.y;
     }
-    __device__ __forceinline__ void operator()(int, cplx<T>&, cplx<T>&) const {}
+    __device__ __forceinline__ void load(int k, const cplx<T>* row, cplx<T>& A, cplx<T>& B) const {
+      A = row[k];
+      B = row[N / 2 + k];
+    }
+    __device__ __forceinline__ void store(int k, cplx<T>* row, cplx<T> A, cplx<T> B) const {
+      row[k] = A;
+      row[N / 2 + k] = B;
+    }
   };
   // the sine series of d/dz when q is given: coefficient k is -q_{N-k} times
   // coefficient N - k, 0 at k = 0
@@ -222,10 +234,10 @@ struct PlaneStages {
       return k == 0 ? mk<T>(T(0), T(0)) : cscale<T>(Planar()(N - k, row), -__ldg(&q[N - k]));
     }
   };
-  // A side <-> Neumann rows one after the other, row pair (2 p, 2 p + 1) at p ld;
-  // ``pairs`` = pair 0, ``c`` = column pair
+  // A side <-> rows one after the other, row pair (2 p, 2 p + 1) at p ld; ``pairs`` =
+  // pair 0, ``c`` = column (Neumann: column pair)
   static __device__ __forceinline__ cplx<T>* planar_at(cplx<T>* pairs, int t, int s, int c, int ld) {
-    const int y = real_pos<N, true>(I::a_elem(t, s));
+    const int y = real_pos<N, DCT>(I::a_elem(t, s));
     return pairs + (y >> 1) * ld + (y & 1) * (N / 2) + c;
   }
   static __device__ __forceinline__ void to_planar(const cplx<T> (&v)[E], int t, cplx<T>* pairs, int c, int ld) {
