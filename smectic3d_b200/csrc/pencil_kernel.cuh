@@ -676,7 +676,10 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
     // The three stress components go forward one after the other, the second and the
     // third on their way into shared memory meanwhile; there the finished spectra
     // take the place of the lines (every thread reads and writes its own slots only).
-    // The projector runs in registers, and the three velocity components go back.
+    // The projector runs in registers, and the three velocity components go back.  1 / |q|^2
+    // is the correctly rounded one: |q|^2 goes with dx^-2 and may be subnormal, where
+    // rcp2 has no value, and the pass waits for memory either way (256^3 FP32 step 819 us
+    // with rcp2, 821 with rcp_rn; Neumann 1004, 1006; FP64 1882, 1905).
     cplx<T>* keep[2] = {aside, aside + size_t(TK) * N};
     constexpr int TH = Cfg::THREADS;
 #pragma unroll
@@ -719,7 +722,7 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
         const cplx<T> px = keep[0][s * TH], py = keep[1][s * TH], pz = v[s];
         // .x holds kz, .y holds kz + 1
         const T m0 = sx * sx + sy * sy + sz0 * sz0, m1 = sx * sx + sy * sy + sz1 * sz1;
-        const T i0 = rcp2(m0), i1 = rcp2(m1);
+        const T i0 = rcp_rn(m0), i1 = rcp_rn(m1);
         const T c0 = scale * ce * i0, c1 = scale * ce * i1;
         const T d0 = sx * px.x + sy * py.x + sz0 * pz.x;
         const T d1 = sx * px.y + sy * py.y + sz1 * pz.y;
@@ -736,7 +739,7 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
         const cplx<T> sx = keep[0][s * TH], sy = keep[1][s * TH], sz = v[s];
         cplx<T> ux = mk<T>(T(0), T(0)), uy = ux, uz = ux;
         if (mq2 != T(0)) {
-          const T inv = rcp2(mq2);
+          const T inv = rcp_rn(mq2);
           const T cm1 = scale * ce * inv;
           const cplx<T> dot = mk<T>(qx * sx.x + qy * sy.x + qz0 * sz.x, qx * sx.y + qy * sy.y + qz0 * sz.y);
           ux = mk<T>(cm1 * (sx.x - qx * inv * dot.x), cm1 * (sx.y - qx * inv * dot.y));
