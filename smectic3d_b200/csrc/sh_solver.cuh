@@ -908,9 +908,12 @@ struct Solver final : SolverBase {
     return capture(kGraphChunk, &graph_exec, &graph_launches);
   }
 
-  // steps outside the kGraphChunk graph
+  // steps outside the kGraphChunk graph; plain launches where the caller captures the stream
   int step_few(int n) {
     if (!many_launches() || !graph_eligible()) return step_direct(n);
+    cudaStreamCaptureStatus capturing;
+    SHB_CUDA(cudaStreamIsCapturing(stream, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone) return step_direct(n);
     int rc;
     const int li = p.l1_interval;
     for (; n > 0; --n) {
