@@ -287,6 +287,59 @@ struct PlaneStages {
       }
     }
   }
+  // The same through the line ``x``, for the 32 values per thread of the split passes:
+  // the lanes of a row pair hold consecutive z and the loops stay rolled.  Unrolled over
+  // the registers, the FP64 code of the sums outgrew the instruction cache, and a store
+  // between two reads of one array kept the reads apart.  256^3 plane pass, us, before ->
+  // now: energy trace, FP32 Neumann 226 -> 113, periodic 144 -> 89, FP64 Neumann 374 ->
+  // 218; L1 monitor every step, 268 -> 146, 1693 -> 135, 428 -> 269.
+  template <class X>
+  static __device__ __forceinline__ void monitor_line(const cplx<T> (&v)[E], int t, const X& x, int flags,
+                                                      const PointParams& pp, int rep, size_t ra, size_t rb,
+                                                      const double* psi_old, double* psi_out, double* o,
+                                                      double* scratch) {
+    x.sync();
+#pragma unroll
+    for (int s = 0; s < E; ++s) x.template store<16>(z_of(t, s), v[s]);
+    x.sync();
+    KahanSum s0, s1, s2;
+    if (flags & kFlL1) {  // all of it before a possibly aliased write
+#pragma unroll 4
+      for (int z = t; z < N; z += I::G) {
+        const cplx<T> q = x.template load<16>(z);
+        const double pa = double(q.x), pb = double(q.y);
+        s0.add(fabs(pa - psi_old[ra + z]) + fabs(pb - psi_old[rb + z]));
+        s1.add(fabs(pa) + fabs(pb));
+      }
+    }
+    if (flags & kFlPsiOut) {
+#pragma unroll 4
+      for (int z = t; z < N; z += I::G) {
+        const cplx<T> q = x.template load<16>(z);
+        psi_out[ra + z] = double(q.x);
+        psi_out[rb + z] = double(q.y);
+      }
+    }
+    if (flags & kFlEnergy) {
+      const double eps = pp.eps[rep];
+#pragma unroll 2
+      for (int z = t; z < N; z += I::G) {
+        const cplx<T> q = x.template load<16>(z);
+        s2.add(local_density(double(q.x), eps, pp.beta, pp.gamma, pp.nonlin) +
+               local_density(double(q.y), eps, pp.beta, pp.gamma, pp.nonlin));
+      }
+    }
+    if (flags & (kFlL1 | kFlEnergy)) {
+      const double t0 = block_sum(s0.s, scratch);
+      const double t1 = block_sum(s1.s, scratch);
+      const double t2 = block_sum(s2.s, scratch);
+      if (threadIdx.x == 0) {
+        o[0] = t0;
+        o[1] = t1;
+        o[2] = t2;
+      }
+    }
+  }
   static __device__ __forceinline__ void real_store(const cplx<T> (&v)[E], int t, T* out, size_t ra, size_t rb) {
 #pragma unroll
     for (int s = 0; s < E; ++s) {

@@ -182,9 +182,9 @@ zrow_kernel(const __grid_constant__ ZrowArgs<T> a) {
   grid_dependency_wait();
   auto monitor = [&] {
     if (a.flags & (kFlPsiOut | kFlL1 | kFlEnergy))
-      S::monitor(v, t, a.flags, a.pp, gp / N, ra, rb, a.psi_old, a.psi_out,
-                 a.red + (size_t(gp) * Cfg::BLOCKS + blockIdx.x % Cfg::BLOCKS) * 3,
-                 reinterpret_cast<double*>(smem_raw + Cfg::RED_OFF));
+      S::monitor_line(v, t, x, a.flags, a.pp, gp / N, ra, rb, a.psi_old, a.psi_out,
+                      a.red + (size_t(gp) * Cfg::BLOCKS + blockIdx.x % Cfg::BLOCKS) * 3,
+                      reinterpret_cast<double*>(smem_raw + Cfg::RED_OFF));
   };
   cplx<T>* keep = reinterpret_cast<cplx<T>*>(smem_raw + Cfg::KEEP_OFF) + threadIdx.x;
   if constexpr (MODE == kZrowStep || MODE == kZrowGen) {
@@ -193,10 +193,11 @@ zrow_kernel(const __grid_constant__ ZrowArgs<T> a) {
     if constexpr (MODE == kZrowGen) {
       monitor();
       if (a.flags & kFlRealOut) S::real_store(v, t, a.real_out, ra, rb);
-      S::nonlin_penalties(v, t, x, a.pp, a.wall, a.lperp, a.kwall, ra, rb);
-    } else {
-      S::nonlin(v, a.pp);
     }
+    if (MODE == kZrowGen && (a.pp.w_mid != 0.0 || a.kwall > 0))
+      S::nonlin_penalties(v, t, x, a.pp, a.wall, a.lperp, a.kwall, ra, rb);
+    else
+      S::nonlin(v, a.pp);
     S::row_forward(v, t, row, x, tw, true, [] {}, typename S::Plain());
   } else if constexpr (MODE == kZrowReal) {
     const int f = blockIdx.y;

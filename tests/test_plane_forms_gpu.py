@@ -1,6 +1,8 @@
 """The forms of the plane pass against one another: one CTA per plane
 (flat_kernel.cuh), clusters (plane_kernel.cuh), one axis at a time
 (split_kernel.cuh)."""
+import time
+
 import numpy as np
 import pytest
 
@@ -35,3 +37,37 @@ def test_one_cta_form_rounds_as_the_clusters(n, cl, boundary, prec):
             assert np.linalg.norm(a - b) <= 1e-14 * np.linalg.norm(b)
         else:
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("boundary", ["periodic", "neumann"])
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+def test_monitors_of_large_planes(boundary, prec):
+    """256^3: the L1 monitor of every step and the energy trace against psi read back,
+    and what they add to a step.  Sums of 1.7e7 terms in FP64, compensated: 1e-12; the
+    trace of an FP32 run takes the gradient part from the new spectrum before it is
+    rounded to real space and back: 1e-6.  The monitor moves two FP64 fields more than
+    the 6 fields of a step (at most 1.7 times the bytes in FP32), the trace none: a
+    step may take 4 and 2 times as long."""
+    n, took = 256, {}
+    kw = dict(n=n, boundary=boundary, precision=prec)
+    for name, extra in (("plain", {}), ("l1", dict(l1_interval=1)), ("trace", dict(energy_trace=True))):
+        with S.Solver(S.Params(**kw, **extra)) as s:
+            s.set_psi(_psi(n))
+            s.step(2)
+            if name == "l1":
+                old = s.get_psi()
+                s.step(1)
+                new = s.get_psi()
+                want = np.abs(new - old).sum() / (s.params.dt * np.abs(new).sum())
+                assert abs(s.l1()[0][0] - want) <= 1e-12 * want
+            if name == "trace":
+                e = s.energy()[0]
+                assert abs(s.energy_trace()[-1] - e) <= (1e-12 if prec == "fp64" else 1e-6) * abs(e)
+            t = []
+            for _ in range(5):
+                t0 = time.perf_counter()
+                s.step(20)
+                t.append(time.perf_counter() - t0)
+            took[name] = min(t)
+    assert took["l1"] <= 4 * took["plain"]
+    assert took["trace"] <= 2 * took["plain"]
