@@ -17,6 +17,8 @@
 // becomes psihat^{n+1} = (W^n + 3 dt/2 Nhat^n) / C2 and
 // W^{n+1} = C1 psihat^{n+1} - dt/2 Nhat^n: one state read and one state write.
 #pragma once
+#include <type_traits>
+
 #include "line_fft.cuh"
 #include "sh_common.cuh"
 
@@ -36,10 +38,11 @@ enum PencilMode : int {
   kPencilAdj = 9,      // adjoint step: lambdahat^n = A lambdahat^{n+1} + ghat^n, mu partial, parameter gradients
   kPencilAdjOut = 10,  // adjoint: lambdahat -> its x-inverse partial (for lambda^0 in real space)
   kPencilStepU64 = 11, // the step of FP32 fields with the CNAB2 multipliers and update in FP64
-  kPencilStepGen = 12, // the step with what kPencilStep leaves out: IMEX Euler, the energy, psihat out
+  kPencilStepGen = 12, // the step with what kPencilStep and kPencilStepEuler leave out: the energy, psihat out
   kPencilStepU64Gen = 13,  // the same for kPencilStepU64
   kPencilStepAdvGen = 14,  // the same for kPencilStepAdv
   kPencilStepSpec = 15,    // kPencilStep that keeps psihat^{n+1} in spec_out (the adjoint's recompute)
+  kPencilStepEuler = 16,   // kPencilStep with IMEX Euler
 };
 // multiplier of kPencilXMul
 enum XMulKind : int {
@@ -240,6 +243,79 @@ __device__ __forceinline__ double rcp2(double x) {
 }
 __device__ __forceinline__ double2 rcp2(double2 x) { return make_double2(rcp2(x.x), rcp2(x.y)); }
 
+// The same where the divisor may overflow: 0 beyond 2^125 (2^1000), as the quotient
+__device__ __forceinline__ float rcp2_or_0(float x) { return fabsf(x) > 0x1p125f ? 0.0f : rcp2(x); }
+__device__ __forceinline__ double rcp2_or_0(double x) { return fabs(x) > 0x1p1000 ? 0.0 : rcp2(x); }
+
+// One mode (Neumann: the pair kz, kz + 1 in .x, .y) of the CNAB2 update:
+//   psihat^{n+1} = (W + 3dt/2 Nhat) / C2,  W' = C1 psihat^{n+1} - dt/2 Nhat
+// h = dt/2, h3 = 3dt/2, qyz = q_y^2 + q_z^2 - q0^2
+template <typename T, bool DCT>
+__device__ __forceinline__ void cnab2_update(T qx, cplx<T> qyz, T alpha, T eps, T h, T h3, cplx<T> nh, cplx<T>& wv,
+                                             cplx<T>& pn) {
+  const cplx<T> d = cfma<T>(both<T>(qx), both<T>(qx), qyz);
+  const cplx<T> al = cfma<T>(cmul2<T>(both<T>(-alpha), d), d, both<T>(eps));
+  const cplx<T> ha = mk<T>(mul_rn(h, al.x), mul_rn(h, al.y));
+  const cplx<T> c2 = csub<T>(both<T>(T(1)), ha), c1 = cadd<T>(both<T>(T(1)), ha);
+  cplx<T> inv;
+  if constexpr (DCT) inv = rcp2(c2);
+  else inv = both<T>(rcp2(c2.x));  // one multiplier for both parts
+  pn = cmul2<T>(cfma<T>(both<T>(h3), nh, wv), inv);
+  wv = cfma<T>(c1, pn, cmul2<T>(both<T>(-h), nh));
+}
+// IMEX Euler: psihat^{n+1} = (psihat + dt Nhat) / (1 - dt aLin),  W' = psihat^{n+1}.
+// Where aLin overflows the mode vanishes (with CNAB2 it is not finite anyway).
+template <typename T, bool DCT>
+__device__ __forceinline__ void euler_update(T qx, cplx<T> qyz, T alpha, T eps, T dt, cplx<T> nh, cplx<T>& wv,
+                                             cplx<T>& pn) {
+  const cplx<T> d = cfma<T>(both<T>(qx), both<T>(qx), qyz);
+  const cplx<T> al = cfma<T>(cmul2<T>(both<T>(-alpha), d), d, both<T>(eps));
+  const cplx<T> c2 = cfma<T>(both<T>(-dt), al, both<T>(T(1)));
+  cplx<T> inv;
+  if constexpr (DCT) inv = mk<T>(rcp2_or_0(c2.x), rcp2_or_0(c2.y));
+  else inv = both<T>(rcp2_or_0(c2.x));
+  pn = cmul2<T>(cfma<T>(both<T>(dt), nh, wv), inv);
+  wv = pn;
+}
+// The same of FP32 fields with the per-mode multipliers and the update in FP64 from
+// the FP64 wavenumbers, one rounding of each stored result.  A multiplier rounded to
+// FP32 repeats the same relative error every step, which drifts a mode's amplitude
+// linearly with the step count.  The products are spelled out so that every kernel
+// rounds alike (a step, a traced step and the adjoint's recompute of it).
+template <typename T, bool DCT>
+__device__ __forceinline__ void cnab2_update64(double qx, double qyz0, double qyz1, double alpha, double eps, double h,
+                                               cplx<T> nh, cplx<T>& wv, cplx<T>& pn) {
+  auto one = [&](double c1, double inv, T n, T& w1, T& p1) {
+    p1 = T((double(w1) + 3.0 * h * double(n)) * inv);
+    w1 = T(fma(c1, double(p1), -__dmul_rn(h, double(n))));
+  };
+  const double e0 = qx * qx + qyz0;
+  const double b0 = eps - alpha * e0 * e0;
+  const double hb0 = __dmul_rn(h, b0), c10 = 1.0 + hb0, i0 = rcp2(1.0 - hb0);
+  double c11 = c10, i1 = i0;
+  if constexpr (DCT) {
+    const double e1 = qx * qx + qyz1;
+    const double b1 = eps - alpha * e1 * e1;
+    const double hb1 = __dmul_rn(h, b1);
+    c11 = 1.0 + hb1;
+    i1 = rcp2(1.0 - hb1);
+  }
+  one(c10, i0, nh.x, wv.x, pn.x);
+  one(c11, i1, nh.y, wv.y, pn.y);
+}
+template <typename T, bool DCT>
+__device__ __forceinline__ void euler_update64(double qx, double qyz0, double qyz1, double alpha, double eps, double dt,
+                                               cplx<T> nh, cplx<T>& wv, cplx<T>& pn) {
+  const double e0 = qx * qx + qyz0, i0 = rcp2_or_0(1.0 - dt * (eps - alpha * e0 * e0));
+  double i1 = i0;
+  if constexpr (DCT) {
+    const double e1 = qx * qx + qyz1;
+    i1 = rcp2_or_0(1.0 - dt * (eps - alpha * e1 * e1));
+  }
+  pn = mk<T>(T((double(wv.x) + dt * double(nh.x)) * i0), T((double(wv.y) + dt * double(nh.y)) * i1));
+  wv = pn;
+}
+
 // What bounds it: Neumann 256^3 FP32 moves 268 MB (41 us at the measured copy
 // rate) in 57 us; 24.0 M warp instructions (41 % of the issue slots), 2.1 M
 // shared-memory wavefronts; the waits are the HBM latency of the line loads and of
@@ -293,19 +369,23 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
   const bool want_energy = (a.flags & kFlEnergy) != 0;
   grid_dependency_wait();
 
-  if constexpr (MODE == kPencilStep || MODE == kPencilStepU64 || MODE == kPencilStepAdv || MODE == kPencilStepSpec) {
-    // CNAB2 and nothing else: this kernel is bound by the instructions it issues
-    // and fetches, so what only some runs ask for (kPencilStepGen) stays out of it
-    cplx<T>* w = a.w + line;
-    Ops::load(v, a.src + line, t);
-    // W is read after the transform: bring its rows (one 128-byte segment per
-    // kx) into L2 meanwhile.  Neumann 256^3 FP32: pencil pass 68.7 -> 64.3 us.
-    // Not for FP64 (137 -> 142 us), nor where the fields live in L2 anyway.
+  // W is read after the transform: bring its rows (one 128-byte segment per kx)
+  // into L2 meanwhile.  Neumann 256^3 FP32: pencil pass 68.7 -> 64.3 us.
+  // Not for FP64 (137 -> 142 us), nor where the fields live in L2 anyway.
+  auto prefetch_w = [&] {
     if constexpr (sizeof(T) == 4 && N >= 256) {
       const cplx<T>* wt = a.w + size_t(rep) * N * FP + f0;
       for (int k = threadIdx.x; k < N; k += Cfg::THREADS)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(wt + size_t(k) * FP));
     }
+  };
+  if constexpr (MODE == kPencilStep || MODE == kPencilStepU64 || MODE == kPencilStepAdv || MODE == kPencilStepSpec ||
+                MODE == kPencilStepEuler) {
+    // One scheme and nothing else: this kernel is bound by the instructions it issues
+    // and fetches, so what only some runs ask for (kPencilStepGen) stays out of it
+    cplx<T>* w = a.w + line;
+    Ops::load(v, a.src + line, t);
+    prefetch_w();
     Ops::forward(v, x, t, tw, false);
     const T q02 = T(a.pp.q0 * a.pp.q0), alpha = T(a.pp.alpha);
     const T h = T(0.5 * a.pp.dt), h3 = T(1.5 * a.pp.dt);
@@ -335,40 +415,12 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
         cplx<T> wv = wreg[i];
         cplx<T> pn;
         if constexpr (MODE == kPencilStepU64) {
-          // FP32 fields with the per-mode multipliers and the update in FP64 from
-          // the FP64 wavenumbers, one rounding of each stored result.  A multiplier
-          // rounded to FP32 repeats the same relative error every step, which
-          // drifts a mode's amplitude linearly with the step count.
           const double qxd = __ldg(&a.qds[t * E + s]);
-          auto update = [&](double qyzd, T n, T& w1, T& p1) {
-            const double e = qxd * qxd + qyzd;
-            const double hb = hd * (epsd - a.pp.alpha * e * e);
-            p1 = T((double(w1) + 3.0 * hd * double(n)) * rcp2(1.0 - hb));
-            w1 = T((1.0 + hb) * double(p1) - hd * double(n));
-          };
-          if constexpr (DCT) {
-            update(qyz0d, nh.x, wv.x, pn.x);
-            update(qyz1d, nh.y, wv.y, pn.y);
-          } else {
-            const double e = qxd * qxd + qyz0d;
-            const double hb = hd * (epsd - a.pp.alpha * e * e), i0 = rcp2(1.0 - hb);
-            pn.x = T((double(wv.x) + 3.0 * hd * double(nh.x)) * i0);
-            pn.y = T((double(wv.y) + 3.0 * hd * double(nh.y)) * i0);
-            wv.x = T((1.0 + hb) * double(pn.x) - hd * double(nh.x));
-            wv.y = T((1.0 + hb) * double(pn.y) - hd * double(nh.y));
-          }
+          cnab2_update64<T, DCT>(qxd, qyz0d, qyz1d, a.pp.alpha, epsd, hd, nh, wv, pn);
+        } else if constexpr (MODE == kPencilStepEuler) {
+          euler_update<T, DCT>(__ldg(&qs[s]), qyz, alpha, eps, T(a.pp.dt), nh, wv, pn);
         } else {
-          const T qx = __ldg(&qs[s]);
-          // .x, .y: kz and kz + 1 (Neumann); one multiplier for both parts (periodic)
-          const cplx<T> d = cfma<T>(both<T>(qx), both<T>(qx), qyz);
-          const cplx<T> al = cfma<T>(cmul2<T>(both<T>(-alpha), d), d, both<T>(eps));
-          const cplx<T> ha = mk<T>(mul_rn(h, al.x), mul_rn(h, al.y));
-          const cplx<T> c2 = csub<T>(both<T>(T(1)), ha), c1 = cadd<T>(both<T>(T(1)), ha);
-          cplx<T> inv;
-          if constexpr (DCT) inv = rcp2(c2);
-          else inv = both<T>(rcp2(c2.x));
-          pn = cmul2<T>(cfma<T>(both<T>(h3), nh, wv), inv);
-          wv = cfma<T>(c1, pn, cmul2<T>(both<T>(-h), nh));
+          cnab2_update<T, DCT>(__ldg(&qs[s]), qyz, alpha, eps, h, h3, nh, wv, pn);
         }
         finite = cfma<T>(pn, both<T>(T(0)), finite);
         if constexpr (MODE == kPencilStepSpec) a.spec_out[line + size_t(Ops::kx_of(t, s)) * FP] = pn;
@@ -380,15 +432,13 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
   } else if constexpr (MODE == kPencilStepGen || MODE == kPencilStepU64Gen || MODE == kPencilStepAdvGen) {
     cplx<T>* w = a.w + line;
     Ops::load(v, a.src + line, t);
+    prefetch_w();
     Ops::forward(v, x, t, tw, false);
-    // mode-independent constants of the update; the (ky, kz) part of |q|^2 is
-    // fixed for the line
     const T q02 = T(a.pp.q0 * a.pp.q0), alpha = T(a.pp.alpha);
     const T h = T(0.5 * a.pp.dt), h3 = T(1.5 * a.pp.dt), dtT = T(a.pp.dt);
     const T qyz0 = qy * qy + qz0 * qz0 - q02;
-    const T qyz1 = qy * qy + qz1 * qz1 - q02;
-    const bool cnab2 = a.pp.scheme == kCNAB2;
-    // FP64 values of the FP32 update (see below); the scalars stay kernel parameters
+    const cplx<T> qyz = mk<T>(qyz0, DCT ? qy * qy + qz1 * qz1 - q02 : qyz0);
+    // FP64 values of the FP32 update; the scalars stay kernel parameters
     const double epsd = a.pp.eps[rep];
     double qyz0d = 0.0, qyz1d = 0.0;
     if constexpr (MODE == kPencilStepU64Gen) {
@@ -399,101 +449,63 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
         qyz1d = qyd * qyd + qz1d * qz1d - a.pp.q0 * a.pp.q0;
       }
     }
-    bool bad = false;
-    // the state W of this line, read after the transform in batches of WB
-    // values: holding all of it through the transform costs the registers of
-    // the resident CTAs
+    cplx<T>* spec = (a.flags & kFlSpecOut) ? a.spec_out + line : nullptr;
+    cplx<T> finite = mk<T>(T(0), T(0));
+    // One loop per scheme, with and without the energy: branches inside one loop kept
+    // the values of a thread apart.  256^3 pencil pass with the energy trace, us, before
+    // -> now: FP32 Neumann 105 -> 84, periodic 74 -> 62, FP64 Neumann 188 -> 156 (IMEX
+    // without it, kPencilStepEuler: 97 -> 78, 68 -> 53, 179 -> 164).
+    auto update = [&](auto cnab2_, auto energy_) {
+      constexpr bool CN = decltype(cnab2_)::value, EN = decltype(energy_)::value;
 #pragma unroll
-    for (int s0 = 0; s0 < E; s0 += WB) {
-      cplx<T> wreg[WB];
+      for (int s0 = 0; s0 < E; s0 += WB) {
+        cplx<T> wreg[WB];
 #pragma unroll
-      for (int i = 0; i < WB; ++i) wreg[i] = w[size_t(Ops::kx_of(t, s0 + i)) * FP];
+        for (int i = 0; i < WB; ++i) wreg[i] = w[size_t(Ops::kx_of(t, s0 + i)) * FP];
 #pragma unroll
-      for (int i = 0; i < WB; ++i) {
-        const int s = s0 + i;
-        const int kx = Ops::kx_of(t, s);
-        const T qx = __ldg(&qs[s]);
-        const T qx2 = qx * qx;
-        cplx<T> wv = wreg[i];
-        const cplx<T> nh = v[s];
-        cplx<T> pn;
-        // psihat^{n+1} = (W + 3dt/2 Nhat) / C2,  W' = C1 psihat^{n+1} - dt/2 Nhat  (CNAB2)
-        // psihat^{n+1} = (psihat + dt Nhat) / (1 - dt aLin),  W' = psihat^{n+1} (IMEX Euler)
-        const T d0 = qx2 + qyz0;
-        const T a0 = eps - alpha * d0 * d0;
-        if constexpr (MODE == kPencilStepU64Gen) {
-          // as kPencilStepU64
-          const double hd = 0.5 * a.pp.dt;
-          const double qxd = __ldg(&a.qds[t * E + s]);
-          const double e0 = qxd * qxd + qyz0d;
-          const double b0 = epsd - a.pp.alpha * e0 * e0;
-          if (cnab2) {
-            const double i0 = 1.0 / (1.0 - hd * b0), c0 = 1.0 + hd * b0;
-            pn.x = T((double(wv.x) + 3.0 * hd * double(nh.x)) * i0);
-            wv.x = T(c0 * double(pn.x) - hd * double(nh.x));
-            double i1 = i0, c1 = c0;
-            if constexpr (DCT) {
-              const double e1 = qxd * qxd + qyz1d;
-              const double b1 = epsd - a.pp.alpha * e1 * e1;
-              i1 = 1.0 / (1.0 - hd * b1);
-              c1 = 1.0 + hd * b1;
+        for (int i = 0; i < WB; ++i) {
+          const int s = s0 + i;
+          const int kx = Ops::kx_of(t, s);
+          const T qx = __ldg(&qs[s]);
+          const cplx<T> nh = v[s];
+          cplx<T> wv = wreg[i], pn;
+          if constexpr (MODE == kPencilStepU64Gen) {
+            const double qxd = __ldg(&a.qds[t * E + s]);
+            if constexpr (CN) cnab2_update64<T, DCT>(qxd, qyz0d, qyz1d, a.pp.alpha, epsd, 0.5 * a.pp.dt, nh, wv, pn);
+            else euler_update64<T, DCT>(qxd, qyz0d, qyz1d, a.pp.alpha, epsd, a.pp.dt, nh, wv, pn);
+          } else {
+            if constexpr (CN) cnab2_update<T, DCT>(qx, qyz, alpha, eps, h, h3, nh, wv, pn);
+            else euler_update<T, DCT>(qx, qyz, alpha, eps, dtT, nh, wv, pn);
+          }
+          if constexpr (EN) {
+            const T qx2 = qx * qx;
+            if constexpr (!DCT) {
+              const double d = double(qx2 + qyz.x);
+              const double wgt = (kz == 0 || kz == N / 2) ? 1.0 : 2.0;
+              acc.add(wgt * d * d * (double(pn.x) * pn.x + double(pn.y) * pn.y));
+            } else {
+              const double wxy = (kx == 0 ? 0.5 : 1.0) * (ky == 0 ? 0.5 : 1.0);
+              const double e0 = double(qx2 + qyz.x), e1 = double(qx2 + qyz.y);
+              acc.add(wxy * ((kz == 0 ? 0.5 : 1.0) * e0 * e0 * double(pn.x) * pn.x + e1 * e1 * double(pn.y) * pn.y));
             }
-            pn.y = T((double(wv.y) + 3.0 * hd * double(nh.y)) * i1);
-            wv.y = T(c1 * double(pn.y) - hd * double(nh.y));
-          } else {
-            const double i0 = 1.0 / (1.0 - a.pp.dt * b0);
-            pn.x = T((double(wv.x) + a.pp.dt * double(nh.x)) * i0);
-            double i1 = i0;
-            if constexpr (DCT) {
-              const double e1 = qxd * qxd + qyz1d;
-              i1 = 1.0 / (1.0 - a.pp.dt * (epsd - a.pp.alpha * e1 * e1));
-            }
-            pn.y = T((double(wv.y) + a.pp.dt * double(nh.y)) * i1);
-            wv = pn;
           }
-        } else if (cnab2) {
-          const T inv0 = rcp_rn(T(1) - h * a0), c10 = T(1) + h * a0;
-          pn.x = (wv.x + h3 * nh.x) * inv0;
-          wv.x = c10 * pn.x - h * nh.x;
-          if constexpr (!DCT) {
-            pn.y = (wv.y + h3 * nh.y) * inv0;
-            wv.y = c10 * pn.y - h * nh.y;
-          } else {
-            const T d1 = qx2 + qyz1;
-            const T a1 = eps - alpha * d1 * d1;
-            const T inv1 = rcp_rn(T(1) - h * a1);
-            pn.y = (wv.y + h3 * nh.y) * inv1;
-            wv.y = (T(1) + h * a1) * pn.y - h * nh.y;
-          }
-        } else {
-          const T inv0 = rcp_rn(T(1) - dtT * a0);
-          pn.x = (wv.x + dtT * nh.x) * inv0;
-          if constexpr (!DCT) {
-            pn.y = (wv.y + dtT * nh.y) * inv0;
-          } else {
-            const T d1 = qx2 + qyz1;
-            pn.y = (wv.y + dtT * nh.y) * rcp_rn(T(1) - dtT * (eps - alpha * d1 * d1));
-          }
-          wv = pn;
+          finite = cfma<T>(pn, both<T>(T(0)), finite);
+          if (spec) spec[size_t(kx) * FP] = pn;
+          w[size_t(kx) * FP] = wv;
+          v[s] = cscale<T>(pn, scale);
         }
-        if (want_energy) {
-          if constexpr (!DCT) {
-            const double d = double(d0);
-            const double wgt = (kz == 0 || kz == N / 2) ? 1.0 : 2.0;
-            acc.add(wgt * d * d * (double(pn.x) * pn.x + double(pn.y) * pn.y));
-          } else {
-            const double wxy = (kx == 0 ? 0.5 : 1.0) * (ky == 0 ? 0.5 : 1.0);
-            const double e0 = double(d0), e1 = double(qx2 + qyz1);
-            acc.add(wxy * ((kz == 0 ? 0.5 : 1.0) * e0 * e0 * double(pn.x) * pn.x + e1 * e1 * double(pn.y) * pn.y));
-          }
-        }
-        bad |= !isfinite(pn.x) || !isfinite(pn.y);
-        if (a.flags & kFlSpecOut) a.spec_out[line + size_t(kx) * FP] = pn;
-        w[size_t(kx) * FP] = wv;
-        v[s] = cscale<T>(pn, scale);
       }
+    };
+    using Yes = std::true_type;
+    using No = std::false_type;
+    if (a.pp.scheme == kCNAB2) {
+      if (want_energy) update(Yes(), Yes());
+      else update(Yes(), No());
+    } else {
+      if (want_energy) update(No(), Yes());
+      else update(No(), No());
     }
-    if (bad) *a.nonfinite = 1;
+    if (!(finite.x == T(0) && finite.y == T(0))) *a.nonfinite = 1;
   } else if constexpr (MODE == kPencilEnergy) {
     // gradient part of the energy of the current state from its partial P,
     // and (kFlShell) its spectral power per |k| shell
@@ -786,7 +798,8 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
     }
   }
 
-  if constexpr (MODE == kPencilStep || MODE == kPencilStepSpec || MODE == kPencilStepGen || MODE == kPencilStepU64 ||
+  if constexpr (MODE == kPencilStep || MODE == kPencilStepSpec || MODE == kPencilStepEuler || MODE == kPencilStepGen ||
+                MODE == kPencilStepU64 ||
                 MODE == kPencilStepU64Gen || MODE == kPencilInit || MODE == kPencilXMul ||
                 MODE == kPencilAdjInit || MODE == kPencilAdj || MODE == kPencilAdjOut) {
     Ops::inverse(v, x, t, tw, MODE != kPencilAdjOut);

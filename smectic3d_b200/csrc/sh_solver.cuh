@@ -310,6 +310,7 @@ struct Solver final : SolverBase {
         return gen ? launch_pencil<kPencilStepU64Gen>(b, reps) : launch_pencil<kPencilStepU64>(b, reps);
     }
     if (p.scheme == kCNAB2 && b.flags == kFlSpecOut) return launch_pencil<kPencilStepSpec>(b, reps);
+    if (p.scheme != kCNAB2 && b.flags == 0) return launch_pencil<kPencilStepEuler>(b, reps);
     if (gen) return launch_pencil<kPencilStepGen>(b, reps);
     return launch_pencil<kPencilStep>(b, reps);
   }
@@ -423,6 +424,7 @@ struct Solver final : SolverBase {
     }
     if ((rc = set_pencil_attrs<kPencilStepGen>())) return rc;
     if ((rc = set_pencil_attrs<kPencilStepSpec>())) return rc;
+    if ((rc = set_pencil_attrs<kPencilStepEuler>())) return rc;
     if ((rc = set_pencil_attrs<kPencilInit>())) return rc;
     if ((rc = set_pencil_attrs<kPencilEnergy>())) return rc;
     if ((rc = set_pencil_attrs<kPencilStepAdv>())) return rc;

@@ -71,3 +71,24 @@ def test_monitors_of_large_planes(boundary, prec):
             took[name] = min(t)
     assert took["l1"] <= 4 * took["plain"]
     assert took["trace"] <= 2 * took["plain"]
+
+
+@pytest.mark.parametrize("advection", [False, True])
+@pytest.mark.parametrize("prec", ["fp32", "fp32_u64", "fp64"])
+@pytest.mark.parametrize("boundary", ["periodic", "neumann"])
+@pytest.mark.parametrize("n", [16, 64, 128])
+def test_a_traced_step_is_the_step(n, boundary, prec, advection):
+    """The kernels with options round every mode as the one without: the energy trace
+    changes no bit of psi, nor (plain steps) of the spectrum W and the partials."""
+    psi, out = _psi(n, 0.8), []
+    kw = dict(n=n, boundary=boundary, precision=prec, advection=advection, dt=0.02)
+    for trace in (False, True):
+        with S.Solver(S.Params(energy_trace=trace, **kw)) as s:
+            s.set_psi(psi)
+            s.step(6)
+            out.append(s.get_psi())
+            if not advection:
+                fields = 3 * n * n * (n // 2 + (boundary == "periodic"))
+                body = s.checkpoint()[-fields * (16 if prec == "fp64" else 8):]
+                out[-1] = out[-1].tobytes() + body
+    assert out[0].tobytes() == out[1].tobytes() if advection else out[0] == out[1]
