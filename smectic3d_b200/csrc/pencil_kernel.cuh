@@ -91,6 +91,8 @@ struct PencilCfg {
     return sizeof(T) == 4 ? (E == 32 ? 384 : (DCT ? 512 : 768)) : (E == 32 ? 256 : 512);
   }
   static constexpr int min_blocks(int mode) {
+    // the six CTAs whose shared memory fits (Neumann 256^3 shells 229 us with five, 198)
+    if (mode == kPencilEnergy && sizeof(T) == 8 && E == 32) return 384 / THREADS;
     return mode != kPencilInit && mode != kPencilInitAdv && mode != kPencilEnergy && step_threads() >= THREADS
                ? step_threads() / THREADS
                : 0;
@@ -519,39 +521,81 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
     // P = IDFT_x(scale psihat): its forward x transform is N scale psihat
     // (REDFT10 after REDFT01: 2N scale psihat)
     const double inv = 1.0 / (a.pp.scale * (DCT ? 2 * N : N));
+    // The spectrum goes through this thread's slots of the exchange tile, so that the
+    // loops stay rolled: their FP64 code for 32 values would fill the instruction
+    // cache.  Periodic: k and N - k, which share |q| and the shell, are added up first.
+    // 256^3, whole calls, us, before -> now: energy FP32 Neumann 181 -> 133, FP64 278 ->
+    // 234 periodic; dominant wavenumber FP64 periodic 208 -> 112.
+    if constexpr (!DCT) Ops::F::canon(v, t);
+    constexpr int NV = DCT ? E : E / 2;  // terms of a thread
+    cplx<T>* own = buf + threadIdx.x;
+    __syncthreads();
 #pragma unroll
-    for (int s = 0; s < E; ++s) {
-      const int kx = Ops::kx_of(t, s);
-      const T qx = __ldg(&qs[s]);
-      const double px = double(v[s].x) * inv, py = double(v[s].y) * inv;
-      const double q02 = double(a.pp.q0) * a.pp.q0;
-      if constexpr (!DCT) {
-        const double d = q02 - double(qx * qx + qy * qy + qz0 * qz0);
-        const double wgt = (kz == 0 || kz == N / 2) ? 1.0 : 2.0;
-        acc.add(wgt * d * d * (px * px + py * py));
+    for (int s = 0; s < E; ++s) own[s * Cfg::THREADS] = v[s];
+    // f(kx, power of kz, power of kz + 1) of term s; periodic: the whole pair's power
+    // as the first, and k = 0 and N / 2, which have no mirror, as two terms
+    auto term = [&](int s, auto f) {
+      const cplx<T> u = own[s * Cfg::THREADS];
+      const double px = double(u.x) * inv, py = double(u.y) * inv;
+      if constexpr (DCT) {
+        f(Ops::kx_of(t, s), px * px, py * py);
       } else {
-        const double wxy = (kx == 0 ? 0.5 : 1.0) * (ky == 0 ? 0.5 : 1.0);
-        const double d0 = q02 - double(qx * qx + qy * qy + qz0 * qz0);
-        const double d1 = q02 - double(qx * qx + qy * qy + qz1 * qz1);
-        acc.add(wxy * ((kz == 0 ? 0.5 : 1.0) * d0 * d0 * px * px + d1 * d1 * py * py));
+        const cplx<T> m = own[(E - 1 - s) * Cfg::THREADS];
+        const double mx = double(m.x) * inv, my = double(m.y) * inv;
+        const double pu = px * px + py * py, pm = mx * mx + my * my;
+        const int k = LineIdx<N>::c_elem(t, s);
+        const bool self = s == 0 && t == 0;
+        f(k < N / 2 ? k : N - k, self ? pu : pu + pm, 0.0);
+        if (s == 0) f(N / 2, self ? pm : 0.0, 0.0);
       }
-      if (want_shell) {
-        // shell = rint |(ix, iy, iz)|: signed indices (Nyquist +N/2) on the periodic
-        // grid, where every kz in (0, N/2) also stands for its conjugate
-        if constexpr (!DCT) {
-          const int ix = kx <= N / 2 ? kx : kx - N, iy = ky <= N / 2 ? ky : ky - N;
-          const int sh = __double2int_rn(sqrt(double(ix * ix + iy * iy + kz * kz)));
-          const double wgt = (kz == 0 || kz == N / 2) ? 1.0 : 2.0;
-          atomicAdd(&hist[sh], wgt * (px * px + py * py));
-        } else {
-          const double wxy = (kx == 0 ? 0.5 : 1.0) * (ky == 0 ? 0.5 : 1.0);
-          const int r2 = kx * kx + ky * ky;
-          const int s0 = __double2int_rn(sqrt(double(r2 + kz * kz)));
-          const int s1 = __double2int_rn(sqrt(double(r2 + (kz + 1) * (kz + 1))));
-          atomicAdd(&hist[s0], wxy * (kz == 0 ? 0.5 : 1.0) * px * px);
-          atomicAdd(&hist[s1], wxy * py * py);
+    };
+    const double wy = ky == 0 ? 0.5 : 1.0, wz = kz == 0 ? 0.5 : 1.0;
+    const double wgt = (kz == 0 || kz == N / 2) ? 1.0 : 2.0;  // periodic: kz also stands for its conjugate
+    if (want_energy) {
+      const double q02 = double(a.pp.q0) * a.pp.q0;
+#pragma unroll 1
+      for (int s = 0; s < NV; ++s)
+        term(s, [&](int kx, double p0, double p1) {
+          const T qx = __ldg(&a.q[kx]);
+          const double d0 = q02 - double(qx * qx + qy * qy + qz0 * qz0);
+          if constexpr (!DCT) {
+            acc.add(wgt * d0 * d0 * p0);
+          } else {
+            const double d1 = q02 - double(qx * qx + qy * qy + qz1 * qz1);
+            acc.add((kx == 0 ? 0.5 : 1.0) * wy * (wz * d0 * d0 * p0 + d1 * d1 * p1));
+          }
+        });
+    }
+    if (want_shell) {
+      // shell = rint |(ix, iy, iz)|: signed indices (Nyquist +N/2) on the periodic
+      // grid.  |.|^2 is below 2^20 and never within 1/4 of (k + 1/2)^2, so FP32 rounds
+      // to the same shell.
+      auto shell = [](int r2) { return __float2int_rn(__fsqrt_rn(float(r2))); };
+      // |k| is monotonic along a tile's lanes, so lanes of one shell are neighbours: the
+      // first adds their sum, instead of all of them meeting at one shared-memory word
+      auto deposit = [&](int sh, double pw) {
+#pragma unroll
+        for (int o = 1; o < TK; o <<= 1) {
+          const int so = __shfl_down_sync(0xffffffffu, sh, o, TK);
+          const double po = __shfl_down_sync(0xffffffffu, pw, o, TK);
+          if (c + o < TK && so == sh) pw += po;
         }
-      }
+        const int left = __shfl_up_sync(0xffffffffu, sh, 1, TK);
+        if (c == 0 || left != sh) atomicAdd(&hist[sh], pw);
+      };
+      const int iy = DCT || ky <= N / 2 ? ky : ky - N;
+#pragma unroll 2
+      for (int s = 0; s < NV; ++s)
+        term(s, [&](int kx, double p0, double p1) {
+          const int r2 = kx * kx + iy * iy;
+          if constexpr (!DCT) {
+            deposit(shell(r2 + kz * kz), wgt * p0);
+          } else {
+            const double wxy = (kx == 0 ? 0.5 : 1.0) * wy;
+            deposit(shell(r2 + kz * kz), wxy * wz * p0);
+            deposit(shell(r2 + (kz + 1) * (kz + 1)), wxy * p1);
+          }
+        });
     }
     if (want_shell) {
       __syncthreads();
