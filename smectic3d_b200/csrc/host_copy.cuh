@@ -17,7 +17,8 @@ namespace shb {
 cudaError_t copy_to_device(void* dst, const void* src, size_t bytes, cudaStream_t stream);
 cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t stream);
 
-// The pinned buffers live from the first large copy to the end of the last handle.
+// Every handle holds the pinned buffers (6 MB, one set per process) while it lives;
+// host_copy.cu says when they are made and given back.
 void host_copy_retain();
 void host_copy_release();
 
