@@ -319,12 +319,93 @@ struct Solver final : SolverBase {
     return launch_pencil<kPencilStepAdv>(b);
   }
 
+  // Raising a kernel's shared-memory limit loads it onto the GPU, about 0.4 ms each the
+  // first time in a process: done for the kernels of the handle's steps when it is
+  // created (a caller may capture them) and for every other at its first launch.
+  // First handle of a process, all kernels -> these: Neumann 256^3 FP32 28 -> 21 ms.
+  bool pencil_used[17] = {}, plane_used[11] = {}, zrow_used[7] = {}, ycol_used[3] = {};
   // a pencil mode whose shared memory does not fit a CTA is never launched
   template <int MODE>
-  int set_pencil_attrs() {
-    if constexpr (QC::fits(MODE)) return set_attrs(pencil_fn<MODE>(), QC::smem(MODE), false);
+  int use_pencil() {
+    if constexpr (QC::fits(MODE)) {
+      if (!pencil_used[MODE])
+        if (const int rc = set_attrs(pencil_fn<MODE>(), QC::smem(MODE), false)) return rc;
+    }
+    pencil_used[MODE] = true;
     return SH_OK;
   }
+  template <int MODE>
+  int use_plane() {
+    if (!plane_used[MODE])
+      if (const int rc = set_attrs(plane_fn<MODE>(), kPlaneSmem, true)) return rc;
+    plane_used[MODE] = true;
+    return SH_OK;
+  }
+  template <int MODE>
+  int use_zrow() {
+    if (!zrow_used[MODE])
+      if (const int rc = set_attrs(&zrow_kernel<T, N, DCT, MODE>, ZC::smem(MODE), false)) return rc;
+    zrow_used[MODE] = true;
+    return SH_OK;
+  }
+  template <bool INV, bool IQY = false>
+  int use_ycol() {
+    constexpr int i = INV ? (IQY ? 2 : 1) : 0;
+    if (!ycol_used[i])
+      if (const int rc = set_attrs(&ycol_kernel<T, N, DCT, INV, IQY>, YC::SMEM, false)) return rc;
+    ycol_used[i] = true;
+    return SH_OK;
+  }
+  // the kernels that set_psi and the steps of this handle launch
+  int use_step_kernels() {
+    int rc = SH_OK;
+    const bool gen = p.scheme != kCNAB2 || p.energy_trace;
+    const bool penalties = kwall > 0 || p.w_mid != 0.0;
+    if (p.advection || kwall > 0) {
+      if ((rc = use_pencil<kPencilInitAdv>())) return rc;
+      if ((rc = gen ? use_pencil<kPencilStepAdvGen>() : use_pencil<kPencilStepAdv>())) return rc;
+      if (p.advection && (rc = use_pencil<kPencilStokes>())) return rc;
+      if ((kwall > 0 || !split()) && (rc = use_plane<kPlaneInvReal>())) return rc;
+    } else {
+      if ((rc = use_pencil<kPencilInit>())) return rc;
+      if (sizeof(T) == 4 && p.precision == SH_FP32_UPDATE64) {
+        if constexpr (sizeof(T) == 4) rc = gen ? use_pencil<kPencilStepU64Gen>() : use_pencil<kPencilStepU64>();
+      } else {
+        rc = p.energy_trace          ? use_pencil<kPencilStepGen>()
+             : p.scheme == kCNAB2 ? use_pencil<kPencilStep>()
+                                  : use_pencil<kPencilStepEuler>();
+      }
+      if (rc) return rc;
+    }
+    if constexpr (kSplit) {
+      if (slab) {
+        if ((rc = use_ycol<true>()) || (rc = use_ycol<false>()) || (rc = use_zrow<kZrowInit>())) return rc;
+        if (!p.advection) {
+          if (!penalties && (rc = use_zrow<kZrowStep>())) return rc;
+          if ((penalties || p.energy_trace || p.l1_interval > 0) && (rc = use_zrow<kZrowGen>())) return rc;
+          return SH_OK;
+        }
+        if constexpr (DCT) {
+          if ((rc = use_zrow<kZrowReal>()) || (rc = use_zrow<kZrowMul>())) return rc;
+        } else {
+          if ((rc = use_ycol<true, true>()) || (rc = use_zrow<kZrowStress>())) return rc;
+        }
+        return use_zrow<kZrowAdvN>();
+      }
+    }
+    if ((rc = use_plane<kPlaneInit>())) return rc;
+    if (p.advection) {
+      if constexpr (DCT) rc = use_plane<kPlaneMulFwd>();
+      else rc = use_plane<kPlaneInvMulFwd>();
+      return rc ? rc : use_plane<kPlaneAdvN>();
+    }
+    if constexpr (kFlat) {
+      if (!penalties && (rc = use_plane<kPlaneStepLean>())) return rc;
+      if (!penalties && !p.energy_trace && p.l1_interval == 0) return SH_OK;
+    }
+    return use_plane<kPlaneStep>();
+  }
+  bool split() const { return kSplit && slab != nullptr; }
 
   int setup() override {
     const size_t fe = field_elems();
@@ -412,54 +493,10 @@ struct Solver final : SolverBase {
     qs = reinterpret_cast<T*>(tables + o_qs);
     qds = reinterpret_cast<double*>(tables + o_qds);
     int rc;
-    if ((rc = set_attrs(plane_fn<kPlaneStep>(), kPlaneSmem, true))) return rc;
-    if ((rc = set_attrs(plane_fn<kPlaneInit>(), kPlaneSmem, true))) return rc;
-    if ((rc = set_attrs(plane_fn<kPlaneGetPsi>(), kPlaneSmem, true))) return rc;
-    if ((rc = set_attrs(plane_fn<kPlaneInvReal>(), kPlaneSmem, true))) return rc;
-    if ((rc = set_pencil_attrs<kPencilStep>())) return rc;
-    if constexpr (sizeof(T) == 4) {
-      if ((rc = set_pencil_attrs<kPencilStepU64>())) return rc;
-      if ((rc = set_pencil_attrs<kPencilStepU64Gen>())) return rc;
-    }
-    if ((rc = set_pencil_attrs<kPencilStepGen>())) return rc;
-    if ((rc = set_pencil_attrs<kPencilStepSpec>())) return rc;
-    if ((rc = set_pencil_attrs<kPencilStepEuler>())) return rc;
-    if ((rc = set_pencil_attrs<kPencilInit>())) return rc;
-    if ((rc = set_pencil_attrs<kPencilEnergy>())) return rc;
-    if ((rc = set_pencil_attrs<kPencilStepAdv>())) return rc;
-    if ((rc = set_pencil_attrs<kPencilStepAdvGen>())) return rc;
-    if ((rc = set_pencil_attrs<kPencilInitAdv>())) return rc;
-    if ((rc = set_pencil_attrs<kPencilStokes>())) return rc;
-    if ((rc = set_pencil_attrs<kPencilXMul>())) return rc;
-    if ((rc = set_pencil_attrs<kPencilSpec>())) return rc;
-    if ((rc = set_pencil_attrs<kPencilAdjInit>())) return rc;
-    if ((rc = set_pencil_attrs<kPencilAdj>())) return rc;
-    if ((rc = set_pencil_attrs<kPencilAdjOut>())) return rc;
-    if ((rc = set_attrs(plane_fn<kPlaneAdj>(), kPlaneSmem, true))) return rc;
-    if ((rc = set_attrs(plane_fn<kPlaneInvMulFwd>(), kPlaneSmem, true))) return rc;
-    if ((rc = set_attrs(plane_fn<kPlaneAdvN>(), kPlaneSmem, true))) return rc;
-    if ((rc = set_attrs(plane_fn<kPlaneMulFwd>(), kPlaneSmem, true))) return rc;
-    if constexpr (kFlat) {
-      if ((rc = set_attrs(plane_fn<kPlaneStepLean>(), kPlaneSmem, true))) return rc;
-      if ((rc = set_attrs(plane_fn<kPlaneStepHist>(), kPlaneSmem, true))) return rc;
-    }
     if constexpr (kSplit) {
-      if ((rc = set_attrs(&ycol_kernel<T, N, DCT, true>, YC::SMEM, false))) return rc;
-      if ((rc = set_attrs(&ycol_kernel<T, N, DCT, false>, YC::SMEM, false))) return rc;
-      if ((rc = set_zrow_attrs<kZrowStep>())) return rc;
-      if ((rc = set_zrow_attrs<kZrowGen>())) return rc;
-      if ((rc = set_zrow_attrs<kZrowAdvN>())) return rc;
-      if ((rc = set_zrow_attrs<kZrowReal>())) return rc;
-      if ((rc = set_zrow_attrs<kZrowInit>())) return rc;
-      if constexpr (DCT) {
-        if ((rc = set_zrow_attrs<kZrowMul>())) return rc;
-      } else {
-        if ((rc = set_attrs(&ycol_kernel<T, N, DCT, true, true>, YC::SMEM, false))) return rc;
-        if ((rc = set_zrow_attrs<kZrowStress>())) return rc;
-      }
       if ((rc = setup_slab())) return rc;
     }
-    return SH_OK;
+    return use_step_kernels();
   }
 
   // The slab of the split passes: whole waves of CTAs, so that no pass ends with a
@@ -473,10 +510,12 @@ struct Solver final : SolverBase {
     long long planes;
     if (p.advection) {
       constexpr int mode = DCT ? int(kZrowAdvN) : int(kZrowStress);
+      if (const int rc = use_zrow<mode>()) return rc;
       SHB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, &zrow_kernel<T, N, DCT, mode>, ZC::THREADS,
                                                              ZC::smem(mode)));
       planes = (long long)occ * sms / ZC::BLOCKS;
     } else {
+      if (const int rc = use_ycol<true>()) return rc;
       SHB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, &ycol_kernel<T, N, DCT, true>, YC::THREADS, YC::SMEM));
       planes = 4ll * occ * sms / YC::TILES;
     }
@@ -491,8 +530,6 @@ struct Solver final : SolverBase {
     slab_planes = int(planes);
     return SH_OK;
   }
-  template <int MODE>
-  int set_zrow_attrs() { return set_attrs(&zrow_kernel<T, N, DCT, MODE>, ZC::smem(MODE), false); }
 
   // one kernel of the split plane pass over ``fields`` fields
   template <class K, class A>
@@ -523,10 +560,14 @@ struct Solver final : SolverBase {
     y.lt = lt;
     y.q = q;
     y.iqy = iqy;
+    int rc;
     if constexpr (!DCT) {
-      if (iqy >= 0)
+      if (iqy >= 0) {
+        if ((rc = use_ycol<true, true>())) return rc;
         return launch_split(&ycol_kernel<T, N, DCT, true, true>, np * YC::TILES, nf, YC::THREADS, YC::SMEM, y);
+      }
     }
+    if ((rc = use_ycol<true>())) return rc;
     return launch_split(&ycol_kernel<T, N, DCT, true>, np * YC::TILES, nf, YC::THREADS, YC::SMEM, y);
   }
   int slab_out(const int* slabs, cplx<T>* const* dst, int nf, size_t p0, int np, int field_planes = 0) {
@@ -536,10 +577,12 @@ struct Solver final : SolverBase {
       y.dst[f] = dst[f] + p0 * FP;
     }
     y.lt = lt;
+    if (const int rc = use_ycol<false>()) return rc;
     return launch_split(&ycol_kernel<T, N, DCT, false>, np * YC::TILES, nf, YC::THREADS, YC::SMEM, y);
   }
   template <int MODE>
   int slab_rows(const ZrowArgs<T>& z, int np, int nf = 1) {
+    if (const int rc = use_zrow<MODE>()) return rc;
     return launch_split(&zrow_kernel<T, N, DCT, MODE>, np * ZC::BLOCKS, nf, ZC::THREADS, ZC::smem(MODE), z);
   }
   cplx<T>* slab_of(int f) const { return slab + size_t(f) * slab_planes * YC::SP; }
@@ -628,6 +671,7 @@ struct Solver final : SolverBase {
       err = "plane pass: unsupported number of argument sets";
       return SH_EINVAL;
     }
+    if (const int rc = use_plane<MODE>()) return rc;
     PlaneLaunch<T> pl{};
     for (int i = 0; i < ncomp; ++i) pl.c[i] = as[i];
     cudaLaunchConfig_t cfg = {};
@@ -658,6 +702,7 @@ struct Solver final : SolverBase {
 
   template <int MODE>
   int launch_pencil(const PencilArgs<T>& a, int reps = 0) {
+    if (const int rc = use_pencil<MODE>()) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(QC::TILES, reps > 0 ? reps : p.batch, 1);
     cfg.blockDim = dim3(QC::THREADS, 1, 1);
@@ -679,6 +724,8 @@ struct Solver final : SolverBase {
     int dev = 0, sms = 0, pb = 0, qb = 0, nc = 0;
     SHB_CUDA(cudaGetDevice(&dev));
     SHB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int rc;
+    if ((rc = use_plane<kPlaneStep>()) || (rc = use_pencil<kPencilStep>())) return rc;
     SHB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pb, plane_fn<kPlaneStep>(), kPlaneThreads, kPlaneSmem));
     SHB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&qb, pencil_fn<kPencilStep>(), QC::THREADS,
                                                            QC::smem(kPencilStep)));
@@ -863,7 +910,6 @@ struct Solver final : SolverBase {
   // costs the GPU about 3 us between kernels (advected 256^3 FP32: 930 us per step
   // launched one by one, 824 replayed): its steps outside the kGraphChunk graph
   // replay a graph of one step.
-  bool split_advected() const { return kSplit && slab != nullptr; }
   bool many_launches() const {
     if constexpr (kSplit) return slab != nullptr && (long long)p.batch * N > slab_planes && !blocked();
     else return false;
@@ -935,7 +981,7 @@ struct Solver final : SolverBase {
   void replayed() {
     if (!p.advection) return;
     real_fields_current = true;
-    lpsi_current = !split_advected() || DCT;
+    lpsi_current = !split() || DCT;
     u_real_current = false;
   }
 
