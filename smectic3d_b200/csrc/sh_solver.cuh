@@ -915,35 +915,40 @@ struct Solver final : SolverBase {
     else return false;
   }
 
-  // capture ``n`` plain steps (nothing runs; the steps counter is restored)
+  // capture ``n`` plain steps.  Nothing runs: what the host notes beside the launches
+  // (counters, which real fields belong to the current state) is as before on return
   int capture(int n, cudaGraphExec_t* exec, long long* count) {
-    cudaGraph_t g;
+    cudaGraph_t g = nullptr;
     const long long s0 = steps, l0 = launches;
+    const int h0 = hist_pos;
+    const bool real0 = real_fields_current, lpsi0 = lpsi_current, u0 = u_real_current;
     // the graph holds plain steps only: the L1 monitor's steps run outside it
     const int li = p.l1_interval;
-    p.l1_interval = 0;
-    SHB_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     int rc = SH_OK;
-    if (blocked()) {
-      for (int r0 = 0; r0 < p.batch && !rc; r0 += p.replica_block) {
-        const int gsz = r0 + p.replica_block <= p.batch ? p.replica_block : p.batch - r0;
-        rc = step_window(r0, gsz, n);
+    cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+      p.l1_interval = 0;
+      if (blocked()) {
+        for (int r0 = 0; r0 < p.batch && !rc; r0 += p.replica_block) {
+          const int gsz = r0 + p.replica_block <= p.batch ? p.replica_block : p.batch - r0;
+          rc = step_window(r0, gsz, n);
+        }
+      } else {
+        rc = step_direct(n);
       }
-      steps += n;
-      hist_pos += n;
-    } else {
-      rc = step_direct(n);
+      p.l1_interval = li;
+      e = cudaStreamEndCapture(stream, &g);
     }
-    cudaError_t e = cudaStreamEndCapture(stream, &g);
-    p.l1_interval = li;
-    steps = s0;
-    hist_pos -= n;
     *count = launches - l0;
+    steps = s0;
     launches = l0;
+    hist_pos = h0;
+    real_fields_current = real0;
+    lpsi_current = lpsi0;
+    u_real_current = u0;
+    if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(exec, g, 0);
+    if (g) cudaGraphDestroy(g);
     if (rc) return rc;
-    SHB_CUDA(e);
-    e = cudaGraphInstantiate(exec, g, 0);
-    cudaGraphDestroy(g);
     SHB_CUDA(e);
     return SH_OK;
   }

@@ -1,4 +1,6 @@
 """Step graphs: the handle's own and the caller's."""
+import threading
+
 import numpy as np
 import pytest
 
