@@ -97,6 +97,7 @@ cudaError_t plain(void* dst, const void* src, size_t bytes, bool to_device, cuda
 }
 
 cudaError_t staged(void* dst, const void* src, size_t bytes, bool to_device, cudaStream_t stream) {
+  if (!dst || !src) return cudaErrorInvalidValue;  // chunks of a null array would have other addresses
   char* host = static_cast<char*>(to_device ? const_cast<void*>(src) : dst);
   char* dev = static_cast<char*>(to_device ? dst : const_cast<void*>(src));
   if (bytes < (to_device ? kMinToDevice : kMinToHost) || !pageable(host)) return plain(dst, src, bytes, to_device, stream);

@@ -1359,7 +1359,19 @@ struct Solver final : SolverBase {
     return SH_OK;
   }
 
-  size_t state_bytes() const override { return (p.advection ? 5 : 3) * field_elems() * sizeof(cplx<T>); }
+  // the fields of a checkpoint after W, P and Nt
+  int advected_fields(cplx<T>* (&f)[2]) const {
+    int n = 0;
+    if (p.advection) {
+      if (!DCT) f[n++] = Px;  // the Neumann gradient is a stencil of psi
+      f[n++] = PSH;
+    }
+    return n;
+  }
+  size_t state_bytes() const override {
+    cplx<T>* f[2];
+    return (3 + advected_fields(f)) * field_elems() * sizeof(cplx<T>);
+  }
   int save_state(void* host) override {
     const size_t fb = field_elems() * sizeof(cplx<T>);
     char* h = static_cast<char*>(host);
@@ -1372,10 +1384,8 @@ struct Solver final : SolverBase {
     SHB_CUDA(copy_to_host(h, wt.p, fb, stream));
     SHB_CUDA(copy_to_host(h + fb, P, fb, stream));
     SHB_CUDA(copy_to_host(h + 2 * fb, Nt, fb, stream));
-    if (p.advection) {
-      SHB_CUDA(copy_to_host(h + 3 * fb, Px, fb, stream));
-      SHB_CUDA(copy_to_host(h + 4 * fb, PSH, fb, stream));
-    }
+    cplx<T>* f[2];
+    for (int i = 0, n = advected_fields(f); i < n; ++i) SHB_CUDA(copy_to_host(h + (3 + i) * fb, f[i], fb, stream));
     SHB_CUDA(cudaStreamSynchronize(stream));
     return SH_OK;
   }
@@ -1391,10 +1401,8 @@ struct Solver final : SolverBase {
     ++launches;
     SHB_CUDA(copy_to_device(P, h + fb, fb, stream));
     SHB_CUDA(copy_to_device(Nt, h + 2 * fb, fb, stream));
-    if (p.advection) {
-      SHB_CUDA(copy_to_device(Px, h + 3 * fb, fb, stream));
-      SHB_CUDA(copy_to_device(PSH, h + 4 * fb, fb, stream));
-    }
+    cplx<T>* f[2];
+    for (int i = 0, n = advected_fields(f); i < n; ++i) SHB_CUDA(copy_to_device(f[i], h + (3 + i) * fb, fb, stream));
     SHB_CUDA(cudaStreamSynchronize(stream));
     ready = true;
     psi0_valid = false;
