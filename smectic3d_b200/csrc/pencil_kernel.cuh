@@ -888,17 +888,17 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
   }
 }
 
-// dst[rep][r][c] -> [rep][c][r] of complex values: the checkpoint file keeps W as
-// [f][kx], the device as [kx][f]
+// src[rep][r][c] -> dst[rep][c - c0][r] of complex values, the columns c0 <= c <
+// c0 + 16 gridDim.x: the checkpoint file keeps W as [f][kx], the device as [kx][f]
 template <typename T>
-__global__ void transpose_kernel(const cplx<T>* __restrict__ src, cplx<T>* __restrict__ dst, int rows, int cols) {
+__global__ void transpose_kernel(const cplx<T>* __restrict__ src, cplx<T>* __restrict__ dst, int rows, int cols,
+                                 int c0) {
   __shared__ cplx<T> tile[16][17];
-  const size_t base = size_t(blockIdx.z) * rows * cols;
   const int c = blockIdx.x * 16 + threadIdx.x, r = blockIdx.y * 16 + threadIdx.y;
-  tile[threadIdx.y][threadIdx.x] = src[base + size_t(r) * cols + c];
+  tile[threadIdx.y][threadIdx.x] = src[(size_t(blockIdx.z) * rows + r) * cols + c0 + c];
   __syncthreads();
   const int c2 = blockIdx.x * 16 + threadIdx.y, r2 = blockIdx.y * 16 + threadIdx.x;
-  dst[base + size_t(c2) * rows + r2] = tile[threadIdx.x][threadIdx.y];
+  dst[(size_t(blockIdx.z) * gridDim.x * 16 + c2) * rows + r2] = tile[threadIdx.x][threadIdx.y];
 }
 
 }  // namespace shb

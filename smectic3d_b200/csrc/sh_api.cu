@@ -517,8 +517,9 @@ int sh_checkpoint_load(sh_handle* h, const void* buf, size_t bytes) {
   std::memcpy(&q, c, sizeof(sh_params));
   if (q.n != s->p.n || q.batch != s->p.batch || q.boundary != s->p.boundary || q.precision != s->p.precision)
     return fail(h, SH_EINVAL, "checkpoint was written by a solver of another shape");
-  std::memcpy(&s->steps, c + sizeof(sh_params), sizeof(long long));
-  return s->load_state(c + sizeof(sh_params) + sizeof(long long));
+  const int rc = s->load_state(c + sizeof(sh_params) + sizeof(long long));
+  if (rc == SH_OK) std::memcpy(&s->steps, c + sizeof(sh_params), sizeof(long long));
+  return rc;
 }
 
 int sh_host_alloc(size_t bytes, void** out) {

@@ -65,13 +65,6 @@ __global__ void to_double_kernel(const T* __restrict__ src, double* __restrict__
 // lowest such shell on a tie)
 __global__ void shell_argmax_kernel(const double* shell, int nshell, double dq, double* out);
 
-// device memory of one call, freed when the call returns
-template <class P>
-struct DeviceScratch {
-  P* p = nullptr;
-  ~DeviceScratch() { cudaFree(p); }
-};
-
 struct SolverBase {
   sh_params p{};
   std::vector<double> eps;
@@ -1372,17 +1365,40 @@ struct Solver final : SolverBase {
     cplx<T>* f[2];
     return (3 + advected_fields(f)) * field_elems() * sizeof(cplx<T>);
   }
+  // columns [f0, f0 + width) of W to their place in the [rep][f][kx] file by way of ``tmp``
+  int transposed_to_host(char* file, cplx<T>* tmp, int f0, int width) {
+    transpose_kernel<T><<<dim3(width / 16, N / 16, p.batch), dim3(16, 16), 0, stream>>>(W, tmp, N, FP, f0);
+    SHB_CUDA(cudaGetLastError());
+    ++launches;
+    constexpr size_t line = N * sizeof(cplx<T>);
+    char* to = file + f0 * line;
+    if (width == FP || p.batch == 1) {
+      SHB_CUDA(copy_to_host(to, tmp, p.batch * width * line, stream));
+    } else {
+      SHB_CUDA(cudaMemcpy2DAsync(to, FP * line, tmp, width * line, width * line, p.batch, cudaMemcpyDeviceToHost, stream));
+      SHB_CUDA(cudaStreamSynchronize(stream));
+    }
+    return SH_OK;
+  }
   int save_state(void* host) override {
     const size_t fb = field_elems() * sizeof(cplx<T>);
     char* h = static_cast<char*>(host);
-    // the file keeps W as [f][kx]
-    DeviceScratch<cplx<T>> wt;
-    SHB_CUDA(dev_malloc(&wt.p, fb));
-    transpose_kernel<T><<<dim3(FP / 16, N / 16, p.batch), dim3(16, 16), 0, stream>>>(W, wt.p, N, FP);
-    SHB_CUDA(cudaGetLastError());
-    ++launches;
-    SHB_CUDA(copy_to_host(h, wt.p, fb, stream));
+    int rc;
     SHB_CUDA(copy_to_host(h + fb, P, fb, stream));
+    // The file keeps W as [f][kx]; it is transposed in memory that the handle has (a
+    // field is 1.1 GB at 512^3 FP64): in d_psi, whose psi^0 is of no use after a step,
+    // or else in P, which then comes back from the file.
+    if (steps == 0 && psi0_valid) {
+      ready = false;
+      if ((rc = transposed_to_host(h, P, 0, FP))) return rc;
+      SHB_CUDA(copy_to_device(P, h + fb, fb, stream));
+      ready = true;
+    } else {
+      constexpr int fits = DCT || sizeof(T) == 4 ? FP : N * (N / 2);  // columns that d_psi holds
+      psi0_valid = false;
+      for (int f0 = 0; f0 < FP; f0 += fits)
+        if ((rc = transposed_to_host(h, reinterpret_cast<cplx<T>*>(d_psi), f0, std::min(fits, FP - f0)))) return rc;
+    }
     SHB_CUDA(copy_to_host(h + 2 * fb, Nt, fb, stream));
     cplx<T>* f[2];
     for (int i = 0, n = advected_fields(f); i < n; ++i) SHB_CUDA(copy_to_host(h + (3 + i) * fb, f[i], fb, stream));
@@ -1393,14 +1409,13 @@ struct Solver final : SolverBase {
     adj_end = -1;
     const size_t fb = field_elems() * sizeof(cplx<T>);
     const char* h = static_cast<const char*>(host);
-    DeviceScratch<cplx<T>> wt;
-    SHB_CUDA(dev_malloc(&wt.p, fb));
-    SHB_CUDA(copy_to_device(wt.p, h, fb, stream));
-    transpose_kernel<T><<<dim3(N / 16, FP / 16, p.batch), dim3(16, 16), 0, stream>>>(wt.p, W, FP, N);
+    ready = false;  // until all of it is there
+    SHB_CUDA(copy_to_device(P, h, fb, stream));
+    transpose_kernel<T><<<dim3(N / 16, FP / 16, p.batch), dim3(16, 16), 0, stream>>>(P, W, FP, N, 0);
     SHB_CUDA(cudaGetLastError());
     ++launches;
-    SHB_CUDA(copy_to_device(P, h + fb, fb, stream));
     SHB_CUDA(copy_to_device(Nt, h + 2 * fb, fb, stream));
+    SHB_CUDA(copy_to_device(P, h + fb, fb, stream));
     cplx<T>* f[2];
     for (int i = 0, n = advected_fields(f); i < n; ++i) SHB_CUDA(copy_to_device(f[i], h + (3 + i) * fb, fb, stream));
     SHB_CUDA(cudaStreamSynchronize(stream));
