@@ -4,7 +4,8 @@ Each built shape offers a few cluster sizes for the plane pass (``variant``):
 - CL = 1 and 2 at 64^3;
 - CL = 1, 2 and 4 at 128^3;
 - CL = 4, 8 and 16 at 256^3 (only for the passes that run clustered there; the
-  steps themselves go one axis at a time and time alike).
+  steps themselves go one axis at a time and time alike, so another size than the
+  default has to be faster by more than such timings differ).
 
 Batched runs of small grids also choose ``replica_block``: how many replicas
 advance together, 16 steps at a time, while their state stays in the 126 MB L2
@@ -20,11 +21,15 @@ boundary, precision, advection), first the cluster size, then the replica
 block with that cluster size, then the pencil tile with both, and keeps the
 fastest. Results are cached in a
 JSON file keyed by that tuple and by the GPU name, under
-$SMECTIC_B200_CACHE (default ~/.cache/smectic3d_b200/tuned.json).
+$SMECTIC_B200_CACHE (default ~/.cache/smectic3d_b200/tuned.json).  An entry that
+was timed with other kernels (a digest of their sources is kept with it) is timed
+again.
 """
 from __future__ import annotations
 
 import dataclasses
+import functools
+import hashlib
 import json
 import os
 import time
@@ -48,6 +53,21 @@ def cache_path() -> Path:
 
 def _key(p, gpu: str) -> str:
     return f"{gpu}|n={p.n}|b={p.batch}|{p.boundary}|{p.precision}|adv={int(bool(p.advection))}"
+
+
+@functools.cache
+def _kernels() -> str:
+    """Digest of the kernel and dispatch sources the library is built from."""
+    h = hashlib.sha256()
+    for f in sorted((Path(__file__).parent / "csrc").glob("*.cu*")):
+        h.update(f.name.encode() + f.read_bytes())
+    return h.hexdigest()[:16]
+
+
+# default cluster size of the sizes whose steps do not depend on it, and the spread of
+# repeated timings of one and the same step (1 to 2 % over 32 steps here)
+_DEFAULT_CL = {256: {"fp64": 16, "fp32": 8, "fp32_u64": 8}}
+_SPREAD = 1.03
 
 
 def _gpu_name() -> str:
@@ -86,7 +106,7 @@ def tune(p, steps: int = 32, use_cache: bool = True) -> dict:
             cache = json.loads(path.read_text())
         except ValueError:
             cache = {}
-    if use_cache and key in cache:
+    if use_cache and cache.get(key, {}).get("kernels") == _kernels():
         return cache[key]
     times = {}
     for v in CANDIDATES.get(p.n, (0,)):
@@ -97,7 +117,10 @@ def tune(p, steps: int = 32, use_cache: bool = True) -> dict:
     if not times:
         raise RuntimeError(f"no plane-pass variant runs for {key}")
     best = min(times, key=times.get)
-    rec = {"variant": best, "us_per_step": {str(k): v for k, v in times.items()}, "replica_block": 0}
+    default = _DEFAULT_CL.get(p.n, {}).get(p.precision)
+    if default in times and times[default] <= _SPREAD * times[best]:
+        best = default
+    rec = {"kernels": _kernels(), "variant": best, "us_per_step": {str(k): v for k, v in times.items()}, "replica_block": 0}
     blocks = [b for b in BLOCKS if b < p.batch] if p.batch > 1 and p.n <= 128 and not p.advection else []
     if blocks:
         bt = {0: times[best]}
