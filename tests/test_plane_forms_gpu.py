@@ -7,6 +7,8 @@ import numpy as np
 import pytest
 
 import smectic3d_b200 as S
+from oracle import sh_oracle as O
+from smectic3d_b200 import _lib as L
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +94,91 @@ def test_a_traced_step_is_the_step(n, boundary, prec, advection):
                 body = s.checkpoint()[-fields * (16 if prec == "fp64" else 8):]
                 out[-1] = out[-1].tobytes() + body
     assert out[0].tobytes() == out[1].tobytes() if advection else out[0] == out[1]
+
+
+def _clustered(monkeypatch, p):
+    """A handle whose slab could not be allocated: its plane passes run clustered."""
+    for k in range(5, 40):
+        monkeypatch.setenv("SMECTIC_B200_TEST_FAIL_ALLOC", str(k))
+        try:
+            s = S.Solver(p)
+        except S.ShError as e:
+            assert e.code == L.SH_ENOMEM
+            continue
+        finally:
+            monkeypatch.delenv("SMECTIC_B200_TEST_FAIL_ALLOC")
+        return s
+    raise AssertionError("no allocation that a handle can do without")
+
+
+def _launches(s):
+    before = s.kernel_launches
+    s.step(1)
+    return s.kernel_launches - before
+
+
+LARGE = [dict(n=256, boundary="periodic"), dict(n=256, boundary="neumann"),
+         dict(n=256, boundary="periodic", w_mid=0.01), dict(n=256, boundary="neumann", w_mid=0.01),
+         dict(n=256, boundary="neumann", sub_sigma=0.5, sub_z0=0.7),
+         dict(n=256, boundary="neumann", nonlinearity="quad_cubic"),
+         dict(n=256, boundary="periodic", scheme="imex_euler"),
+         dict(n=256, boundary="periodic", advection=True, dt=0.02, w_mid=0.01),
+         dict(n=256, boundary="neumann", advection=True, dt=0.02, w_mid=0.01)]
+
+
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-12), ("fp32", 2e-6)])
+@pytest.mark.parametrize("kw", LARGE, ids=str)
+def test_split_passes_match_the_clusters(monkeypatch, kw, prec, tol):
+    """256^3 with each option, one axis at a time against clusters of the default size:
+    psi^0 and its N, three steps with the monitor, the energy.  A step is some 50
+    dependent roundings of 1.1e-16 or 6e-8 on terms of the size of psi, the sums of the
+    monitor and the energy less: 1e-12 and 2e-6 after three steps, ten times that with
+    the advected step's products of derivatives."""
+    tol *= 10 if kw.get("advection") else 1
+    psi, out = _psi(256, 0.8), []
+    p = S.Params(precision=prec, l1_interval=2, **kw)
+    for make in (lambda: S.Solver(p), lambda: _clustered(monkeypatch, p)):
+        with make() as s:
+            s.set_psi(psi)
+            first = _launches(s)
+            s.step(2)
+            out.append([first, s.get_psi(), s.l1()[0], np.array(s.energy())])
+    assert out[1][0] < out[0][0]  # fewer launches: the second handle did run clustered
+    for a, b in zip(out[0][1:], out[1][1:]):
+        assert np.linalg.norm(a - b) <= tol * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("n,boundary,cl", [(256, "neumann", 4), (256, "periodic", 16), (512, "neumann", 16),
+                                           (512, "periodic", 16)])
+def test_every_cluster_size_still_steps(monkeypatch, n, boundary, cl):
+    """The other cluster sizes of 256^3 and the 512^3 planes (clusters of 16, direct
+    exchange), FP32, as above."""
+    psi, out = _psi(n, 0.8), []
+    p = S.Params(n=n, boundary=boundary, precision="fp32", variant=cl)
+    for make in (lambda: S.Solver(p), lambda: _clustered(monkeypatch, p)):
+        with make() as s:
+            s.set_psi(psi)
+            first = _launches(s)
+            s.step(2)
+            out.append((first, s.get_psi()))
+    assert out[1][0] < out[0][0]
+    assert np.linalg.norm(out[0][1] - out[1][1]) <= 2e-6 * np.linalg.norm(out[1][1])
+
+
+@pytest.mark.parametrize("kw", [dict(boundary="periodic", w_mid=0.01, nonlinearity="quad_cubic"),
+                                dict(boundary="neumann", sub_sigma=0.5, sub_z0=0.7),
+                                dict(boundary="neumann", w_mid=0.01, scheme="imex_euler")], ids=str)
+def test_options_of_large_planes_match_the_oracle(kw):
+    """256^3 FP64, two steps (the second takes N of a state the kernels made)."""
+    n = 256
+    p = S.Params(n=n, precision="fp64", **kw)
+    psi = _psi(n, 0.8)
+    op = O.Params(n=n, dx=p.dx, dt=p.dt, eps=p.eps, nonlinearity=p.nonlinearity, scheme=p.scheme, w_mid=p.w_mid,
+                  sub_sigma=p.sub_sigma, sub_z0=p.sub_z0)
+    o = (O.PeriodicOracle if p.boundary == "periodic" else O.NeumannOracle)(psi, op)
+    o.run(2)
+    with S.Solver(p) as s:
+        s.set_psi(psi)
+        s.step(2)
+        out = s.get_psi()
+    assert np.linalg.norm(out - o.psi) <= 1e-12 * np.linalg.norm(o.psi)
