@@ -218,11 +218,12 @@ __device__ __forceinline__ float2 cmul2<float>(float2 a, float2 b) {
 // products that no addition may absorb (ptxas fuses a packed mul and add)
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-// Reciprocals of the step's C2 (a normal number for every step that keeps psi
-// finite).  FP32: the hardware approximation and one Newton-Raphson iteration
-// r + r (1 - x r) in fused arithmetic; __frcp_rn, whose value it is for every
-// significand and the exponents from 2^-27 to 2^36 (checked over all of
-// them), carries a branch to a subnormal path in every use.
+// Reciprocals of the step's divisors C2 = 1 -+ (a rounded product), which are 0 (then
+// psi turns non-finite with any reciprocal) or at least 2^-24 in size, 2^-53 in FP64.
+// FP32: the hardware approximation and one Newton-Raphson iteration r + r (1 - x r) in
+// fused arithmetic; equal to __frcp_rn for every significand from 2^-24 to 2^125, above
+// which the approximation is flushed to 0 (NaN at infinity; C1 is infinite there too).
+// With __frcp_rn the pencil pass takes 73.5 us instead of 64.5 at Neumann 256^3.
 __device__ __forceinline__ float rcp2(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -236,7 +237,7 @@ __device__ __forceinline__ float2 rcp2(float2 x) {
   return cfma<float>(r, e, r);
 }
 // FP64: the 20-bit approximation and two iterations (relative error 2^-80 before
-// the last rounding)
+// the last rounding), 2^-53 to 2^1000
 __device__ __forceinline__ double rcp2(double x) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
