@@ -1,6 +1,9 @@
 // Staged host copies (host_copy.cuh).
 #include "host_copy.cuh"
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <chrono>
 #include <cstdint>
@@ -13,10 +16,12 @@ namespace {
 
 constexpr int kWorkers = 6;               // memcpy threads; 6 x 8 GB/s is about the link rate
 constexpr size_t kChunk = size_t(1) << 19;  // per buffer, two buffers per worker: 6 MB pinned in all
-// Below these the threads cost more than they save.  To the device 17 MB take 850 us
-// plain and 680 staged; to the host 17 MB 960 and 980, 134 MB 7.8 ms and 5.5 (27.9 and
-// 9.6 into untouched pages).
-constexpr size_t kMinToDevice = size_t(4) << 20, kMinToHost = size_t(32) << 20;
+// Below kMin the threads cost more than they save: to the device 17 MB take 850 us plain
+// and 680 staged.  To the host 17 MB take 850 us plain and 650 to 1100 staged when the
+// array's pages exist, but 3 ms more plain when they do not (the page faults, which the
+// threads share): staged from kMinToHost on (134 MB 7.8 -> 5.5 ms), below that only into
+// untouched pages (adjoint of 128^3, T = 400: 24.6 -> 22.1 ms).
+constexpr size_t kMin = size_t(4) << 20, kMinToHost = size_t(32) << 20;
 // Making and freeing the buffers takes 6.6 ms here (2.5 even for 64 KB) and a staged
 // copy saves some 85 us per MB: they are made once the plain copies since the last
 // time would have paid for them, and freed with the last handle unless a copy went
@@ -48,6 +53,18 @@ bool pageable(const void* host) {
     return true;
   }
   return at.type == cudaMemoryTypeUnregistered;
+}
+
+// whether most of the array's pages were never touched, by a sample of eight
+bool untouched(const char* host, size_t bytes) {
+  const uintptr_t page = uintptr_t(sysconf(_SC_PAGESIZE));
+  int n = 0;
+  for (int i = 0; i < 8; ++i) {
+    const uintptr_t at = (reinterpret_cast<uintptr_t>(host) + (2 * i + 1) * (bytes / 16)) & ~(page - 1);
+    unsigned char in_memory = 1;
+    if (mincore(reinterpret_cast<void*>(at), page, &in_memory) == 0 && !(in_memory & 1)) ++n;
+  }
+  return n >= 4;
 }
 
 // worker w of n: chunks w, w + n, ... through its two buffers
@@ -100,7 +117,7 @@ cudaError_t staged(void* dst, const void* src, size_t bytes, bool to_device, cud
   if (!dst || !src) return cudaErrorInvalidValue;  // chunks of a null array would have other addresses
   char* host = static_cast<char*>(to_device ? const_cast<void*>(src) : dst);
   char* dev = static_cast<char*>(to_device ? dst : const_cast<void*>(src));
-  if (bytes < (to_device ? kMinToDevice : kMinToHost) || !pageable(host)) return plain(dst, src, bytes, to_device, stream);
+  if (bytes < kMin || !pageable(host) || (!to_device && bytes < kMinToHost && !untouched(host, bytes))) return plain(dst, src, bytes, to_device, stream);
   Pool& p = pool();
   std::unique_lock<std::mutex> lock(p.use, std::try_to_lock);
   if (!lock.owns_lock()) return plain(dst, src, bytes, to_device, stream);
