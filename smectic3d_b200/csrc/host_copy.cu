@@ -16,12 +16,15 @@ namespace {
 
 constexpr int kWorkers = 6;               // memcpy threads; 6 x 8 GB/s is about the link rate
 constexpr size_t kChunk = size_t(1) << 19;  // per buffer, two buffers per worker: 6 MB pinned in all
-// Below kMin the threads cost more than they save: to the device 17 MB take 850 us plain
-// and 680 staged.  To the host 17 MB take 850 us plain and 650 to 1100 staged when the
-// array's pages exist, but 3 ms more plain when they do not (the page faults, which the
-// threads share): staged from kMinToHost on (134 MB 7.8 -> 5.5 ms), below that only into
-// untouched pages (adjoint of 128^3, T = 400: 24.6 -> 22.1 ms).
-constexpr size_t kMin = size_t(4) << 20, kMinToHost = size_t(32) << 20;
+// Below kMin the threads cost more than they save: 17 MB to the device take 820 us plain
+// and 640 staged, but three fields of 8 MB only 0.1 ms less, and an array that the caller
+// frees after other threads have touched it is slower to unmap (Solver.restore of a
+// Neumann 128^3 FP32 handle 3.4 ms plain, 4.2 staged).
+// To the host 17 MB take 850 us plain and 650 to 1100 staged when the array's pages
+// exist, but 3 ms more plain when they do not (the page faults, which the threads share):
+// staged from kMinToHost on (134 MB 7.8 -> 5.5 ms), below that only into untouched pages
+// (adjoint of 128^3, T = 400: 24.6 -> 22.1 ms).
+constexpr size_t kMin = size_t(12) << 20, kMinToHost = size_t(32) << 20;
 // Making and freeing the buffers takes 6.6 ms here (2.5 even for 64 KB) and a staged
 // copy saves some 85 us per MB: they are made once the plain copies since the last
 // time would have paid for them, and freed with the last handle unless a copy went
