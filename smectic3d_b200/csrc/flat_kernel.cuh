@@ -37,10 +37,11 @@ struct FlatCfg {
   static constexpr int MIN_BLOCKS = THREADS <= STEP_THREADS ? STEP_THREADS / THREADS : 1;
 };
 
-// What bounds it: 64 x 64^3 FP32 the shared-memory pipe (81 % busy, 12 moves of the
-// plane; 54 us for 134 MB), 128^3 FP64 its barriers and the one CTA of 16 warps that
-// an SM holds (23 us).  The step's plane pass before -> now: 64 x 64^3 FP32 periodic
-// 85 -> 54 us, Neumann 99 -> 58; 128^3 FP32 20.9 -> 14.8, FP64 25.6 -> 23.1.
+// What bounds it: 64 x 64^3 FP32 the shared-memory pipe (79 % busy, 12 moves of the
+// plane; 51 us for 134 MB), 128^3 FP64 its barriers and the one CTA of 16 warps that
+// an SM holds (22 us).  The step's plane pass, event to event, plane_kernel -> now:
+// 64 x 64^3 FP32 periodic 84.1 -> 52.0 us, Neumann 98.5 -> 56.9; periodic 128^3 FP32
+// 20.5 -> 14.3, FP64 26.5 -> 22.2.
 template <typename T, int N, bool DCT, int MODE>
 __global__ void __launch_bounds__(FlatCfg<T, N, DCT>::THREADS,
                                   MODE == kPlaneStepLean || MODE == kPlaneStepHist || MODE == kPlaneAdj

@@ -320,14 +320,15 @@ __device__ __forceinline__ void euler_update64(double qx, double qyz0, double qy
 }
 
 // What bounds it: Neumann 256^3 FP32 moves 268 MB (41 us at the measured copy
-// rate) in 57 us; 24.0 M warp instructions (41 % of the issue slots), 2.1 M
+// rate) in 55 us; 24.5 M warp instructions (45 % of the issue slots), 2.1 M
 // shared-memory wavefronts; the waits are the HBM latency of the line loads and of
 // W.  The 16-values-per-thread form it replaces staged tiles in shared memory and
 // paired k with N - k by shuffles: 42 M instructions, 7.5 M wavefronts, 76 us.
-// Step pencil pass, before -> now: periodic 256^3 FP32 64.8 -> 57.3, Neumann 256^3
-// FP64 153 -> 137, Neumann 512^3 FP64 1672 -> 1180, periodic 512^3 FP32 637 -> 469,
-// periodic 128^3 FP64 23.1 -> 16.8, 64 x 64^3 FP32 68.7 -> 52.8 periodic, 83.3 -> 57.0
-// Neumann, FP64 update (kPencilStepU64) Neumann 256^3 95 -> 79 us.
+// Step pencil pass, event to event, that form -> now: Neumann 256^3 FP32 76.3 -> 61.1,
+// periodic 65.3 -> 54.8, Neumann 256^3 FP64 154 -> 143, Neumann 512^3 FP64 1716 -> 1138,
+// periodic 512^3 FP32 634 -> 470, periodic 128^3 FP64 23.3 -> 16.6, 64 x 64^3 FP32 68.9
+// -> 52.9 periodic, 84.0 -> 57.9 Neumann, FP64 update (kPencilStepU64) Neumann 256^3
+// 95.7 -> 72.1 us.
 template <typename T, int N, bool DCT, int MODE, int TKV = 0>
 __global__ void __launch_bounds__(PencilCfg<T, N, DCT, TKV>::THREADS, PencilCfg<T, N, DCT, TKV>::min_blocks(MODE))
 pencil_kernel(const __grid_constant__ PencilArgs<T> a) {

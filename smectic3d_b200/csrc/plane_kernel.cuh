@@ -24,7 +24,8 @@
 //
 // This form serves 16^2 planes, the cluster sizes a handle asks for, and at 256^2
 // and 512^2 the modes that split_kernel.cuh does not have; flat_kernel.cuh takes
-// planes of 32^2 to 128^2 with one CTA (64 x 64^3 FP32 step pass 85 -> 54 us).
+// planes of 32^2 to 128^2 with one CTA (64 x 64^3 FP32 step pass 84 -> 52 us), and at
+// 256^2 and 512^2 all modes of a handle whose slab could not be allocated.
 #pragma once
 #include "sh_common.cuh"
 

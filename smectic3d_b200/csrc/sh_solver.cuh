@@ -247,9 +247,10 @@ struct Solver final : SolverBase {
   size_t field_elems() const { return size_t(p.batch) * N * FP; }
 
   // Planes too large for one CTA go through the split passes (256^3 Neumann FP32 step
-  // 170 us clustered, 131 split; 512^3 FP64 6580, 2670).  Where a plane fits a CTA the
-  // one-CTA kernel is faster than three passes (128^3 FP64 27.6 us per step against
-  // 34.4, 64 x 64^3 FP32 95 against 120).
+  // 170 us clustered, 127 split; 512^3 FP64 6580, 2680; advected 256^3 FP32 periodic 965,
+  // 821, Neumann 1086, 1017, FP64 periodic 2437, 1878).  Where a plane fits a CTA the
+  // one-CTA kernel is faster than three passes (128^3 FP64 26.1 us per step against
+  // 34.4, 64 x 64^3 FP32 93 against 120; advected steps there were not tried split).
   static constexpr bool kSplit = N >= 256;
   using YC = YcolCfg<T, N, DCT>;
   using ZC = ZrowCfg<T, N, DCT>;
@@ -272,7 +273,7 @@ struct Solver final : SolverBase {
   }
 
   // Planes that fit one CTA run in the one-CTA form (64 x 64^3 FP32 step 133 us with
-  // plane_kernel, 95 with flat_kernel; 128^3 FP32 21.1, 15.0)
+  // plane_kernel, 93 with flat_kernel; 128^3 FP32 21.1, 15.3)
   using LC = FlatCfg<T, N, DCT>;
   static constexpr bool kFlat = CL == 1 && LC::ok;
   static constexpr int kPlaneThreads = kFlat ? LC::THREADS : PC::THREADS;
@@ -292,8 +293,8 @@ struct Solver final : SolverBase {
     return SH_OK;
   }
 
-  // The kernel without options wherever none is asked for (Neumann 256^3 FP32 69 us,
-  // with them as branches 92).  The plain step's pencil pass: FP32 fields take their CNAB2 multipliers in
+  // The kernel without options wherever none is asked for (Neumann 256^3 FP32 61 us;
+  // kPencilStepGen with the energy 84).  FP32 fields take their CNAB2 multipliers in
   // FP64 when the handle asks for it (SH_FP32_UPDATE64)
   int launch_pencil_step(const PencilArgs<T>& b, int reps = 0) {
     const bool gen = p.scheme != kCNAB2 || b.flags != 0;
@@ -515,7 +516,8 @@ struct Solver final : SolverBase {
     planes = std::max(1ll, std::min(planes, (long long)p.batch * N));
     const size_t bytes = size_t(planes) * YC::SP * sizeof(cplx<T>) * (p.advection ? kSplitComps : 1);
     if (dev_malloc(&slab, bytes) != cudaSuccess) {
-      // the fields themselves fit: keep the clustered plane pass, which needs no slab
+      // the fields themselves fit: keep the clustered plane pass, which needs no slab but
+      // takes up to 2.4 times as long per step (two launches instead of four tell)
       cudaGetLastError();
       slab = nullptr;
       return SH_OK;
@@ -902,7 +904,9 @@ struct Solver final : SolverBase {
   // A step that goes slab by slab is 21 to 60 launches, and outside a graph each
   // costs the GPU about 3 us between kernels (advected 256^3 FP32: 930 us per step
   // launched one by one, 824 replayed): its steps outside the kGraphChunk graph
-  // replay a graph of one step.
+  // replay a graph of one step.  Steps of two launches do not: ten steps of 32^3 FP64
+  // take 74 us launched and 77 replayed (64^3 Neumann FP32 105, 117), and recording the
+  // graph costs 90 us once; a single step alone would gain (26 us, 19).
   bool many_launches() const {
     if constexpr (kSplit) return slab != nullptr && (long long)p.batch * N > slab_planes && !blocked();
     else return false;

@@ -7,7 +7,7 @@ import smectic3d_b200 as S
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [32, 128])  # 128: fields above the 4 MB that are staged by threads
+@pytest.mark.parametrize("n", [32, 128])  # 128 FP64: fields large enough to be staged by threads
 @pytest.mark.parametrize("prec", ["fp32", "fp64"])
 @pytest.mark.parametrize("boundary", ["periodic", "neumann"])
 def test_advected_checkpoint_round_trip(boundary, prec, n):

@@ -31,3 +31,18 @@ def test_short_lived_handles_do_not_pay_for_the_staging_buffers():
 
     best(pageable)
     assert best(pageable) <= best(pinned) + 4e-3
+
+
+@pytest.mark.parametrize("n,b", [(32, 47), (32, 129), (64, 6)])
+def test_staged_arrays_cross_unchanged(n, b):
+    """12.3 and 33.8 MB, whose last chunk of 512 KB is half one, and 12.6 MB: psi^0 comes
+    back as it went in, through the driver and (after 64 MB of copies) through the
+    staging buffers, into new arrays and into one that is used again."""
+    psi = np.random.default_rng(n + b).uniform(-1, 1, size=(b, n, n, n))
+    out = np.empty_like(psi)
+    with S.Solver(S.Params(n=n, batch=b, precision="fp64")) as s:
+        for k in range(12):
+            a = psi + k
+            s.set_psi(a)
+            assert np.array_equal(s.get_psi(), a)
+            assert np.array_equal(s.run(a, 0, out), a)

@@ -182,3 +182,36 @@ def test_options_of_large_planes_match_the_oracle(kw):
         s.step(2)
         out = s.get_psi()
     assert np.linalg.norm(out - o.psi) <= 1e-12 * np.linalg.norm(o.psi)
+
+
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-11), ("fp32", 1e-5)])
+def test_adjoint_of_large_planes_matches_a_small_box(prec, tol):
+    """256^3: states that repeat every 64 points have the repeated gradient of the 64^3
+    box and 64 times its parameter gradients.  The reverse sweep's planes run clustered,
+    the recomputed steps one axis at a time; 7 steps out and back are some 700 roundings."""
+    psi, out = _psi(64), {}
+    for n, p in ((64, "fp64"), (256, prec)):
+        with S.Solver(S.Params(n=n, precision=p)) as s:
+            s.adjoint_forward(np.tile(psi, (n // 64,) * 3), 7, 3)
+            end = s.get_psi()
+            out[n] = [end, *s.adjoint_backward(end - 0.5)]
+    for i, scale in ((0, 1), (3, 1), (1, 64), (2, 64)):
+        want = scale * (np.tile(out[64][i], (4, 4, 4)) if i in (0, 3) else out[64][i])
+        assert np.linalg.norm(out[256][i] - want) <= tol * np.linalg.norm(want), i
+
+
+@pytest.mark.parametrize("curvature", ["difference", "spectral"])
+def test_curvature_pass_of_large_planes(monkeypatch, curvature):
+    """Neumann 256^3 FP64: the curvature pass on a state the split passes made against
+    the one that the clusters made (1e-12 of psi; divided by gradients of order 0.1)."""
+    psi, out = S.ic.hyperboloid(256, 2 * np.pi / 8, amp=1.3, r0_cells=20, seed=1), []
+    p = S.Params(n=256, boundary="neumann", precision="fp64", curvature=curvature)
+    for make in (lambda: S.Solver(p), lambda: _clustered(monkeypatch, p)):
+        with make() as s:
+            s.set_psi(psi)
+            s.step(2)
+            out.append(s.surface_step())
+    assert (out[0][0] >= 0).any() and np.array_equal(out[0][0], out[1][0])
+    for a, b in zip(out[0][1:], out[1][1:]):
+        assert np.array_equal(np.isnan(a), np.isnan(b))
+        assert np.linalg.norm(np.nan_to_num(a - b)) <= 1e-9 * np.linalg.norm(np.nan_to_num(b))
