@@ -573,17 +573,20 @@ pencil_kernel(const __grid_constant__ PencilArgs<T> a) {
       // grid.  |.|^2 is below 2^20 and never within 1/4 of (k + 1/2)^2, so FP32 rounds
       // to the same shell.
       auto shell = [](int r2) { return __float2int_rn(__fsqrt_rn(float(r2))); };
-      // |k| is monotonic along a tile's lanes, so lanes of one shell are neighbours: the
-      // first adds their sum, instead of all of them meeting at one shared-memory word
+      // |k| is monotonic along the lanes of one ky row (or half the kz = N/2 column), so
+      // those of one shell are neighbours: the first adds their sum, instead of all of
+      // them meeting at one shared-memory word
+      constexpr int W = TK < N / 2 ? TK : N / 2;  // a tile of 16^3 holds two rows
+      const int cw = c % W;
       auto deposit = [&](int sh, double pw) {
 #pragma unroll
-        for (int o = 1; o < TK; o <<= 1) {
-          const int so = __shfl_down_sync(0xffffffffu, sh, o, TK);
-          const double po = __shfl_down_sync(0xffffffffu, pw, o, TK);
-          if (c + o < TK && so == sh) pw += po;
+        for (int o = 1; o < W; o <<= 1) {
+          const int so = __shfl_down_sync(0xffffffffu, sh, o, W);
+          const double po = __shfl_down_sync(0xffffffffu, pw, o, W);
+          if (cw + o < W && so == sh) pw += po;
         }
-        const int left = __shfl_up_sync(0xffffffffu, sh, 1, TK);
-        if (c == 0 || left != sh) atomicAdd(&hist[sh], pw);
+        const int left = __shfl_up_sync(0xffffffffu, sh, 1, W);
+        if (cw == 0 || left != sh) atomicAdd(&hist[sh], pw);
       };
       const int iy = DCT || ky <= N / 2 ? ky : ky - N;
 #pragma unroll 2
