@@ -36,3 +36,28 @@ def test_a_few_steps_can_be_captured_by_the_caller(kw):
             g.replay()
             g.replay()
         assert np.array_equal(a.get_psi(), b.get_psi())
+
+
+@pytest.mark.parametrize("n", [32, 256])
+def test_prepare_leaves_a_restored_state_to_be_computed(n):
+    """sh_prepare records the step graph and changes no state: the velocity and the
+    surface pass of a restored checkpoint are those without it (the real-space fields
+    they read belong to the handle's state before, or to none)."""
+    kw = dict(n=n, precision="fp32", advection=True, dt=0.02)
+    with S.Solver(S.Params(**kw)) as s:
+        s.set_psi(_psi(n))
+        s.step(3)
+        blob = s.checkpoint()
+    out = {}
+    for prepare in (False, True):
+        for what in ("velocity", "surface_step"):
+            with S.Solver(S.Params(**kw)) as s:
+                s.set_psi(S.ic.noise(n, 5, 0.3))
+                s.step(1)
+                s.restore(blob)
+                if prepare:
+                    s.prepare()
+                out[prepare, what] = getattr(s, what)()
+    for what in ("velocity", "surface_step"):
+        for a, b in zip(out[False, what], out[True, what]):
+            assert np.array_equal(a, b, equal_nan=True)
