@@ -350,7 +350,7 @@ struct Solver final : SolverBase {
     ycol_used[i] = true;
     return SH_OK;
   }
-  // the kernels that set_psi and the steps of this handle launch
+  // the kernels that set_psi, the steps and get_psi of this handle launch
   int use_step_kernels() {
     int rc = SH_OK;
     const bool gen = p.scheme != kCNAB2 || p.energy_trace;
@@ -374,20 +374,21 @@ struct Solver final : SolverBase {
     if constexpr (kSplit) {
       if (slab) {
         if ((rc = use_ycol<true>()) || (rc = use_ycol<false>()) || (rc = use_zrow<kZrowInit>())) return rc;
+        if ((rc = use_zrow<kZrowReal>())) return rc;
         if (!p.advection) {
           if (!penalties && (rc = use_zrow<kZrowStep>())) return rc;
           if ((penalties || p.energy_trace || p.l1_interval > 0) && (rc = use_zrow<kZrowGen>())) return rc;
           return SH_OK;
         }
         if constexpr (DCT) {
-          if ((rc = use_zrow<kZrowReal>()) || (rc = use_zrow<kZrowMul>())) return rc;
+          if ((rc = use_zrow<kZrowMul>())) return rc;
         } else {
           if ((rc = use_ycol<true, true>()) || (rc = use_zrow<kZrowStress>())) return rc;
         }
         return use_zrow<kZrowAdvN>();
       }
     }
-    if ((rc = use_plane<kPlaneInit>())) return rc;
+    if ((rc = use_plane<kPlaneInit>()) || (rc = use_plane<kPlaneGetPsi>())) return rc;
     if (p.advection) {
       if constexpr (DCT) rc = use_plane<kPlaneMulFwd>();
       else rc = use_plane<kPlaneInvMulFwd>();

@@ -61,3 +61,34 @@ def test_prepare_leaves_a_restored_state_to_be_computed(n):
     for what in ("velocity", "surface_step"):
         for a, b in zip(out[False, what], out[True, what]):
             assert np.array_equal(a, b, equal_nan=True)
+
+
+@pytest.mark.parametrize("kw", [dict(n=32), dict(n=128, boundary="neumann", sub_sigma=0.5), dict(n=64, variant=2),
+                                dict(n=256, precision="fp64"), dict(n=64, advection=True, dt=0.02),
+                                dict(n=256, boundary="neumann", advection=True, dt=0.02),
+                                dict(n=256, scheme="imex_euler", w_mid=0.01)], ids=str)
+def test_a_new_handle_can_be_captured(kw):
+    """The first calls of a handle, psi in, steps and psi out on the device, recorded by
+    the caller before any kernel of it has run."""
+    import torch
+
+    p = S.Params(**{"precision": "fp32", **kw})
+    with S.Solver(p) as a, S.Solver(p) as b:
+        psi = torch.tensor(_psi(p.n), device="cuda")
+        out, want = torch.zeros_like(psi), torch.zeros_like(psi)
+        torch.cuda.synchronize()
+        st = torch.cuda.ExternalStream(a.stream)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(st):
+            g.capture_begin()
+            a.set_psi_device(psi.data_ptr())
+            a.step_async(2)
+            a.get_psi_device(out.data_ptr())
+            g.capture_end()
+            g.replay()
+        a.synchronize()
+        b.set_psi_device(psi.data_ptr())
+        b.step(2)
+        b.get_psi_device(want.data_ptr())
+        b.synchronize()
+        assert torch.equal(out, want) and float(want.abs().max()) > 0.1
