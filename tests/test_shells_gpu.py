@@ -29,7 +29,7 @@ def _flat(n, boundary, k, seed):
     scale[k] *= np.sqrt(1.02)
     scale[0] = 0.0
     spec = spec * scale[shell]
-    y = np.fft.irfftn(spec, (n, n, n)) if boundary == "periodic" else O.idct3d(spec)
+    y = np.fft.irfftn(spec, (n, n, n), axes=(0, 1, 2)) if boundary == "periodic" else O.idct3d(spec)
     return y / np.abs(y).max()
 
 
